@@ -42,27 +42,27 @@ def listed():
       name=name, model=model, dtype=dtype, kind=kind, batch=batch, low=low, high=high, new=new, slots=slots, burst=burst)
   return [
       # A short question: the whole model for a handful of tokens, where launches and the host count.
-      case("prompt 13, 2B", "gemma2-2b", "prompt", 1, 13, 13),
+      case("prompt 13 2B", "gemma2-2b", "prompt", 1, 13, 13),
       # The ordinary prompt of one request, the size the benchmark prints.
-      case("prompt 2048, 2B", "gemma2-2b", "prompt", 1, 2048, 2048),
+      case("prompt 2048 2B", "gemma2-2b", "prompt", 1, 2048, 2048),
       # Requests of all lengths that arrive together and share a step.
-      case("prompts together, 2B", "gemma2-2b", "prompt", 7, 3, 1500),
+      case("prompts together 2B", "gemma2-2b", "prompt", 7, 3, 1500),
       # A document for the larger model: the largest step.
-      case("prompt 3001, 9B", "gemma2-9b", "prompt", 1, 3001, 3001),
+      case("prompt 3001 9B", "gemma2-9b", "prompt", 1, 3001, 3001),
       # One user's tokens, one after the other: latency.
-      case("decode 1, 2B", "gemma2-2b", "decode", 1, 700, 1100),
+      case("decode 1 2B", "gemma2-2b", "decode", 1, 700, 1100),
       # The benchmark's headline: eight requests near the longest context.
-      case("decode 8 long, 2B", "gemma2-2b", "decode", 8, 7040, 7168),
+      case("decode 8 long 2B", "gemma2-2b", "decode", 8, 7040, 7168),
       # Serving: requests of all sizes come and go, prompts beside decoded tokens in one step.
-      case("serve 64, 2B", "gemma2-2b", "generate", 64, 24, 640, new=64, slots=40, burst=4),
+      case("serve 64 2B", "gemma2-2b", "generate", 64, 24, 640, new=64, slots=40, burst=4),
       # The 32-bit path, which users take to check results: a text's likelihood.
       case("score 301 in float32", "gemma2 2b-like", "score", 1, 301, 301, dtype="float32"),
       # Routed experts and a gated recurrence: a prompt, and eight users.
-      case("prompt 2048, experts", "sapivik 2b-like", "prompt", 1, 2048, 2048),
-      case("decode 8, experts", "sapivik 2b-like", "decode", 8, 500, 1500),
+      case("prompt 2048 experts", "sapivik 2b-like", "prompt", 1, 2048, 2048),
+      case("decode 8 experts", "sapivik 2b-like", "decode", 8, 500, 1500),
       # Latent attention, delta rule, state space: two prompts of odd lengths, and eight users.
-      case("prompts 2, latent", "zesapel 2b-like", "prompt", 2, 517, 1531),
-      case("decode 8, latent", "zesapel 2b-like", "decode", 8, 500, 1500),
+      case("prompts 2 latent", "zesapel 2b-like", "prompt", 2, 517, 1531),
+      case("decode 8 latent", "zesapel 2b-like", "decode", 8, 500, 1500),
   ]
 
 
