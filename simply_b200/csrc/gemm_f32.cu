@@ -1,72 +1,264 @@
 // True 32-bit matrix product on CUDA cores: out[M, N] = x[M, K] . w[N, K]^T.
 //
 // No tensor-core mode, no reduced-precision staging: every product and sum is a
-// float32 FMA.  The sum over K runs in the same order for every row whatever M
-// is, so a token's result does not depend on what else is in the batch.
+// float32 FMA.  Every output is one chain of FMAs over k = 0, 1, ..., K - 1, whatever tile
+// computes it, so a token's result does not depend on what else is in the batch.
 // Optional epilogue: soft cap (simply/model_lib.py:107-109) for the output layer.
+//
+// Bound by the FMA pipes for many rows, by the weights' bytes for a few.  Three tile shapes share the
+// chains' order: 64 x 64 outputs (8 x 4 per thread, packed FMAs) where those fill the GPU, 32 x 32
+// (4 x 2 per thread) where they do not, and 16 x 16 fed by a deep ring of asynchronous copies for
+// up to 16 rows, where the weights only stream by.
 #include "common.cuh"
 
-#define BM 64
-#define BN 64
-#define BK 16
+// Two FMAs in one instruction, each rounded as fmaf rounds.
+__device__ __forceinline__ void fma_pair(float2& acc, float2 a, float2 b) {
+  unsigned long long* c = reinterpret_cast<unsigned long long*>(&acc);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;"
+      : "+l"(*c)
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+}
 
-__global__ void __launch_bounds__(256) gemm_f32_nt_kernel(const float* __restrict__ x,
-                                                          const float* __restrict__ w,
-                                                          float* __restrict__ out, int M, int N, int K,
-                                                          float cap) {
+__device__ __forceinline__ float capped(float v, float cap) { return cap > 0.f ? cap * tanhf(v / cap) : v; }
+
+// Four values of a row from k on (zeros beyond the matrix); `vec`: rows start on 16-byte boundaries.
+__device__ __forceinline__ float4 row_quad(const float* __restrict__ p, bool in, int k, int K, bool vec) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!in) return v;
+  if (vec) {
+    if (k < K) v = *reinterpret_cast<const float4*>(p + k);
+  } else {
+    if (k < K) v.x = p[k];
+    if (k + 1 < K) v.y = p[k + 1];
+    if (k + 2 < K) v.z = p[k + 2];
+    if (k + 3 < K) v.w = p[k + 3];
+  }
+  return v;
+}
+
+// ---------------------------------------------------------------------------
+// Many rows: a BM x BN tile, TM x TN outputs per thread as TM / 2 pairs of rows.  Tiles of BK k stand
+// turned round in shared memory ([k][row], so a thread reads its rows as one vector), twice: while
+// one is multiplied the next one's values are on their way in registers.  Neighbouring lanes fetch a
+// row's 16-byte quads; the rows of the four k of quad q are kept at places row ^ turn(q), so that the
+// 32 values a warp stores at a time lie on 32 banks.
+//
+// What bounds it: a warp's reads of shared memory deliver 128 bytes a cycle and SM, so TM + TN cycles per
+// k beside TM TN / 4 cycles of FMAs: 16 x 8 outputs per thread keep the FMA pipes the longer of the two,
+// 8 x 8 are even, and 8 x 4 are half as long again as their FMAs (taken where larger tiles would leave SMs idle).
+// ---------------------------------------------------------------------------
+template <int BM, int BN, int BK, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out, int M, int N,
+                     int K, float cap, int vec) {
+  constexpr int THREADS = (BM / TM) * (BN / TN), QUADS = BK / 4;
+  constexpr int XQ = BM * QUADS / THREADS, WQ = BN * QUADS / THREADS;  // quads a thread fetches per tile
+  static_assert(BM * QUADS % THREADS == 0 && BN * QUADS % THREADS == 0, "whole quads per thread");
+  static_assert(TM % 4 == 0 && TN % 4 == 0 && QUADS <= 8 && BM % 32 == 0 && BN % 32 == 0, "vectors of 4, places within a row");
   pdl_wait_block();
   pdl_launch_dependents();
-  __shared__ float xs[BK][BM + 1];
-  __shared__ float ws[BK][BN + 1];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  __shared__ __align__(16) float xs[2][BK][BM];
+  __shared__ __align__(16) float ws[2][BK][BN];
+  // A warp is 4 groups of rows by 8 of columns: its vectors of a k are few and shared.
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int WARP_COLS = BN / (8 * TN);
+  // (a thread's columns: groups of 4, 32 apart, so that 8 lanes read 128 bytes in a row)
+  const int mt = ((warp / WARP_COLS) * 4 + (lane >> 3)) * TM, nt = (warp % WARP_COLS) * 8 * TN + (lane & 7) * 4;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    // 64 rows x 16 columns per operand: 1024 values, 4 per thread.
+  const int quad = threadIdx.x % QUADS, row = threadIdx.x / QUADS;
+  auto turn = [](int q) { return (q % 4) * 8 + (q / 4) * 4; };
+  constexpr int STEP = THREADS / QUADS;  // rows between a thread's pieces
+  float4 xq[XQ], wq[WQ];
+  auto fetch = [&](int k0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int idx = threadIdx.x + i * 256;
-      const int r = idx / BK, c = idx % BK;
-      const int gm = m0 + r, gn = n0 + r, gk = k0 + c;
-      xs[c][r] = (gm < M && gk < K) ? x[(size_t)gm * K + gk] : 0.f;
-      ws[c][r] = (gn < N && gk < K) ? w[(size_t)gn * K + gk] : 0.f;
+    for (int i = 0; i < XQ; ++i) {
+      const int r = m0 + row + i * STEP;
+      xq[i] = row_quad(x + (size_t)r * K, r < M, k0 + quad * 4, K, vec);
     }
-    __syncthreads();
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = xs[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = ws[k][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    for (int i = 0; i < WQ; ++i) {
+      const int r = n0 + row + i * STEP;
+      wq[i] = row_quad(w + (size_t)r * K, r < N, k0 + quad * 4, K, vec);
     }
+  };
+  auto put = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < XQ; ++i) {
+      const int r = (row + i * STEP) ^ turn(quad);
+      xs[buf][quad * 4][r] = xq[i].x; xs[buf][quad * 4 + 1][r] = xq[i].y; xs[buf][quad * 4 + 2][r] = xq[i].z; xs[buf][quad * 4 + 3][r] = xq[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < WQ; ++i) {
+      const int r = (row + i * STEP) ^ turn(quad);
+      ws[buf][quad * 4][r] = wq[i].x; ws[buf][quad * 4 + 1][r] = wq[i].y; ws[buf][quad * 4 + 2][r] = wq[i].z; ws[buf][quad * 4 + 3][r] = wq[i].w;
+    }
+  };
+  float2 acc[TM / 2][TN];
+#pragma unroll
+  for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  fetch(0);
+  put(0);
+  __syncthreads();
+  for (int k0 = 0, buf = 0; k0 < K; k0 += BK, buf ^= 1) {
+    const bool more = k0 + BK < K;
+    if (more) fetch(k0 + BK);
+    float2 a[2][TM / 2];
+    float b[2][TN];
+    auto read = [&](int s, int k) {
+      const int at = turn(k / 4);
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&xs[buf][k][(mt + i) ^ at]);
+        a[s][i / 2] = make_float2(v.x, v.y);
+        a[s][i / 2 + 1] = make_float2(v.z, v.w);
+      }
+#pragma unroll
+      for (int j = 0; j < TN; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&ws[buf][k][(nt + j * 8) ^ at]);
+        b[s][j] = v.x; b[s][j + 1] = v.y; b[s][j + 2] = v.z; b[s][j + 3] = v.w;
+      }
+    };
+    read(0, 0);
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {  // (values beyond K are zeros on both sides: the chain keeps its value)
+      if (k + 1 < BK) read((k + 1) & 1, k + 1);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        const float2 bb = make_float2(b[k & 1][j], b[k & 1][j]);
+#pragma unroll
+        for (int i = 0; i < TM / 2; ++i) fma_pair(acc[i][j], a[k & 1][i], bb);
+      }
+    }
+    if (more) put(buf ^ 1);
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty * 4 + i;
-    if (gm >= M) continue;
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + mt + i;
+    if (gm >= M) break;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + tx * 4 + j;
-      if (gn >= N) continue;
-      float v = acc[i][j];
-      if (cap > 0.f) v = cap * tanhf(v / cap);
-      out[(size_t)gm * N + gn] = v;
+    for (int j = 0; j < TN; ++j) {
+      const int gn = n0 + nt + (j / 4) * 32 + j % 4;
+      if (gn < N) out[(size_t)gm * N + gn] = capped(i & 1 ? acc[i / 2][j].y : acc[i / 2][j].x, cap);
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// Up to 16 rows: one output per thread, 128 per block (ROWS x 128 / ROWS).  The weights' rows stream
+// through a ring of asynchronous 16-byte copies (rows of 16-byte multiples only), several blocks per
+// SM; the chain of one output (4 cycles per k) is what is left, so a thread has the vectors of the
+// next 16 k in registers while it multiplies these.
+// ---------------------------------------------------------------------------
+#define F32_FEW 16        // most rows
+#define F32_FEW_K 128     // k per stage
+#define F32_FEW_STAGES 5
+#define F32_FEW_LD (F32_FEW_K + 4)  // a row's start moves on by 4 banks
+
+template <int ROWS>
+__global__ void __launch_bounds__(128)
+gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out, int M, int N, int K,
+                    float cap) {
+  constexpr int COLS = 128 / ROWS, STAGE = (COLS + ROWS) * F32_FEW_LD, PIECES = F32_FEW_K / 4;
+  extern __shared__ __align__(16) float few_smem[];  // stages of (weights [COLS][LD], x [ROWS][LD])
+  const int n0 = blockIdx.x * COLS;
+  const int steps = (K + F32_FEW_K - 1) / F32_FEW_K;
+  // A warp copies a row's 512 bytes at a time.  (Beyond the matrix: 0 bytes read, zeros written.)
+  const int piece = (threadIdx.x % PIECES) * 4, first = threadIdx.x / PIECES;
+  auto copy = [&](const float* from, int rows, int count, int step, float* to) {
+    const int k = step * F32_FEW_K + piece;
+    for (int r = first; r < count; r += 128 / PIECES) {
+      const bool in = r < rows && k < K;
+      const float* src = in ? from + (size_t)r * K + k : from;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(to + r * F32_FEW_LD + piece)), "l"(src), "r"(in ? 16 : 0));
+    }
+  };
+  const float* wn = w + (size_t)n0 * K;
+  // The weights of the first stages need nothing from the kernel before.
+  for (int s = 0; s < F32_FEW_STAGES - 1; ++s)
+    if (s < steps) copy(wn, N - n0, COLS, s, few_smem + s * STAGE);
+  pdl_wait_block();
+  pdl_launch_dependents();
+  for (int s = 0; s < F32_FEW_STAGES - 1; ++s) {
+    if (s < steps) copy(x, M, ROWS, s, few_smem + s * STAGE + COLS * F32_FEW_LD);
+    asm volatile("cp.async.commit_group;\n");
+  }
+  const int m = threadIdx.x / COLS, n = threadIdx.x % COLS;
+  float acc = 0.f;
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(F32_FEW_STAGES - 2));
+    __syncthreads();  // the stage has landed for all; the one read a turn ago is free
+    const int next = s + F32_FEW_STAGES - 1;
+    if (next < steps) {
+      float* to = few_smem + (next % F32_FEW_STAGES) * STAGE;
+      copy(wn, N - n0, COLS, next, to);
+      copy(x, M, ROWS, next, to + COLS * F32_FEW_LD);
+    }
+    asm volatile("cp.async.commit_group;\n");
+    const float* wr = few_smem + (s % F32_FEW_STAGES) * STAGE + n * F32_FEW_LD;
+    const float* xr = few_smem + (s % F32_FEW_STAGES) * STAGE + (COLS + m) * F32_FEW_LD;
+    if (m < M) {
+      float4 a[2][4], b[2][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        a[0][q] = *reinterpret_cast<const float4*>(xr + 4 * q);
+        b[0][q] = *reinterpret_cast<const float4*>(wr + 4 * q);
+      }
+#pragma unroll
+      for (int k = 0; k < F32_FEW_K; k += 16) {
+        const int at = (k / 16) & 1;
+        if (k + 16 < F32_FEW_K) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            a[at ^ 1][q] = *reinterpret_cast<const float4*>(xr + k + 16 + 4 * q);
+            b[at ^ 1][q] = *reinterpret_cast<const float4*>(wr + k + 16 + 4 * q);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          acc = fmaf(a[at][q].x, b[at][q].x, acc);
+          acc = fmaf(a[at][q].y, b[at][q].y, acc);
+          acc = fmaf(a[at][q].z, b[at][q].z, acc);
+          acc = fmaf(a[at][q].w, b[at][q].w, acc);
+        }
+      }
+    }
+  }
+  if (m < M && n0 + n < N) out[(size_t)m * N + n0 + n] = capped(acc, cap);
+}
+
+template <int ROWS>
+static int launch_f32_few(const float* x, const float* w, float* out, int M, int N, int K, float cap, cudaStream_t stream) {
+  constexpr int COLS = 128 / ROWS;
+  constexpr size_t smem = (size_t)F32_FEW_STAGES * (COLS + ROWS) * F32_FEW_LD * sizeof(float);
+  const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  sb_launch_early(gemm_f32_few_kernel<ROWS>, (N + COLS - 1) / COLS, 128, smem, stream, x, w, out, M, N, K, cap);
+  SB_LAUNCH_CHECK();
+  return 0;
+}
+
+template <int BM, int BN, int BK, int TM, int TN>
+static int launch_f32_tile(const float* x, const float* w, float* out, int M, int N, int K, float cap, int vec,
+                           cudaStream_t stream) {
+  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+  if (grid.y > 65535) return -6;
+  sb_launch(gemm_f32_tile_kernel<BM, BN, BK, TM, TN>, grid, (BM / TM) * (BN / TN), 0, stream, x, w, out, M, N, K, cap, vec);
+  SB_LAUNCH_CHECK();
+  return 0;
 }
 
 extern "C" int sb_gemm_f32_nt(const float* x, const float* w, float* out, int M, int N, int K, float cap,
                               cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) return -6;
-  sb_launch(gemm_f32_nt_kernel, grid, 256, 0, stream, x, w, out, M, N, K, cap);
-  SB_LAUNCH_CHECK();
-  return 0;
+  const int vec = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+  if (M <= F32_FEW && vec && K > 0)
+    return M <= 8 ? launch_f32_few<8>(x, w, out, M, N, K, cap, stream) : launch_f32_few<16>(x, w, out, M, N, K, cap, stream);
+  auto tiles = [&](int bm, int bn) { return (long long)((N + bn - 1) / bn) * ((M + bm - 1) / bm); };
+  if (tiles(128, 128) >= 200) return launch_f32_tile<128, 128, 16, 16, 8>(x, w, out, M, N, K, cap, vec, stream);
+  if (tiles(64, 64) >= 96) return launch_f32_tile<64, 64, 32, 8, 4>(x, w, out, M, N, K, cap, vec, stream);
+  return launch_f32_tile<32, 32, 32, 4, 4>(x, w, out, M, N, K, cap, vec, stream);
 }

@@ -211,6 +211,21 @@ def test_linear_float32_is_true_float32(table, m, n, k):
   assert torch.equal(alone[0], got[m // 2])
 
 
+# (rows around those of the kernel for a few rows, and sizes on both sides of each tile shape's rule)
+@pytest.mark.parametrize("m,n,k,shift", [(8, 33, 36, 0), (9, 20, 132, 0), (16, 17, 520, 0), (16, 40, 128, 1), (17, 31, 16, 0),
+                                         (65, 3100, 31, 0), (70, 3100, 100, 0), (260, 9000, 20, 0), (130, 13000, 17, 3)])
+def test_linear_float32_row_is_the_same_in_every_tile(table, m, n, k, shift):
+  ops = table[torch.float32]
+  x = torch.randn(m, k, device="cuda")
+  w = torch.randn(n * k + shift, device="cuda")[shift:].view(n, k)  # (a weight need not start on 16 bytes)
+  got = ops.linear(x, w)
+  # k roundings of partial sums of about sqrt(k) each, 2^-24 of it at most
+  assert (got.double() - x.double() @ w.double().t()).abs().max() < 8 * k * 2.0 ** -24
+  for row in (0, m // 2, m - 1):
+    assert torch.equal(ops.linear(x[row:row + 1], w)[0], got[row])
+  assert torch.equal(ops.linear(x, w[:5])[:, :5], got[:, :5])
+
+
 @pytest.mark.parametrize("m", [1, 3, 8, 9, 16, 17, 24, 32, 33, 47, 64, 65, 200])
 @pytest.mark.parametrize("n,k", [(48, 64), (1000, 96), (2304, 2048), (100, 328), (130, 9216), (4096, 2304)])
 def test_linear_bfloat16(table, m, n, k):
