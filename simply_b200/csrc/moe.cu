@@ -1,4 +1,4 @@
-// Feed-forward layers made of routed experts.  Five kernels, none of which needs the host to
+// Feed-forward layers made of routed experts.  None of the kernels needs the host to
 // know how the tokens were dealt out, so a step can be captured in a CUDA graph:
 //
 //   route    per token: router logits z = W_r x (+ a learned offset per expert) (float32), scores
@@ -13,11 +13,13 @@
 //   combine  y[t] = sum_j weight[t, j] * (expert output of pair (t, j), or x[t] for an identity
 //            expert) + gate[t] * shared[t], summed in the order of j
 //
-// bfloat16 products run on tensor cores (mma.sync through nvcuda::wmma) with float32 sums; the
-// float32 path uses CUDA cores only.  A row's result does not depend on which rows share its tile.
+// The products here serve float32 (CUDA cores only) and bfloat16 widths that are no multiple of 8
+// (mma.sync through nvcuda::wmma, float32 sums); other bfloat16 products are in moe_tc.cu.  A row's
+// result does not depend on which rows share its tile.
 #include <mma.h>
 
 #include "common.cuh"
+#include "moe_activation.cuh"
 
 #define MOE_TILE_M 64   // rows of a tile
 #define MOE_TILE_N 32   // output columns of one set of weight rows
@@ -158,14 +160,18 @@ extern "C" int sb_moe_route(const void* x, int dtype, int num_tokens, int width,
 
 // ---------------------------------------------------------------------------
 // group: one block.  P pairs (pair p = token p / top, choice p % top), E experts with rows.
-//   sorted_pair [P]: the pairs of expert 0, then of expert 1, ... (unused entries at the end: -1)
+//   sorted_pair [P]: the pairs of expert 0, then of expert 1, ... (`padded`: an expert's pairs begin at a
+//                    multiple of tile_m; entries between are not written)
 //   pos_of_pair [P]: where pair p stands in sorted_pair, or -1 for an identity expert's pair
 //   tile_expert / tile_row0 / tile_rows [max_tiles]: the tiles; unused ones have expert -1
+//   tile_count: how many tiles there are; `padded`: tile_row0 is the first tile of the tile's expert, and
+//                    tile_span how many its expert has
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024)
 moe_group_kernel(const int* __restrict__ chosen, int P, int E, int max_tiles, int* __restrict__ sorted_pair,
                  int* __restrict__ pos_of_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
-                 int* __restrict__ tile_rows) {
+                 int* __restrict__ tile_rows, int* __restrict__ tile_span, int* __restrict__ tile_count, int tile_m,
+                 int padded) {
   pdl_wait_block();
   pdl_launch_dependents();
   extern __shared__ int group_smem[];  // counts [E], offsets [E], tile_base [E], cursor [E]
@@ -184,19 +190,21 @@ moe_group_kernel(const int* __restrict__ chosen, int P, int E, int max_tiles, in
   if (threadIdx.x == 0) {
     int rows = 0, tiles = 0;
     for (int e = 0; e < E; ++e) {
-      offsets[e] = rows;
+      offsets[e] = padded ? tiles * tile_m : rows;
       tile_base[e] = tiles;
       rows += counts[e];
-      tiles += (counts[e] + MOE_TILE_M - 1) / MOE_TILE_M;
+      tiles += (counts[e] + tile_m - 1) / tile_m;
     }
+    *tile_count = tiles;
   }
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     const int n = counts[e];
-    for (int i = 0, k = tile_base[e]; i < n && k < max_tiles; i += MOE_TILE_M, ++k) {
+    for (int i = 0, k = tile_base[e]; i < n && k < max_tiles; i += tile_m, ++k) {
       tile_expert[k] = e;
-      tile_row0[k] = offsets[e] + i;
-      tile_rows[k] = min(MOE_TILE_M, n - i);
+      tile_row0[k] = padded ? tile_base[e] : offsets[e] + i;
+      if (padded) tile_span[k] = (n + tile_m - 1) / tile_m;
+      tile_rows[k] = min(tile_m, n - i);
     }
   }
   for (int p = threadIdx.x; p < P; p += blockDim.x) {
@@ -211,12 +219,14 @@ moe_group_kernel(const int* __restrict__ chosen, int P, int E, int max_tiles, in
 }
 
 extern "C" int sb_moe_group(const int* chosen, int P, int E, int max_tiles, int* sorted_pair, int* pos_of_pair,
-                            int* tile_expert, int* tile_row0, int* tile_rows, cudaStream_t stream) {
+                            int* tile_expert, int* tile_row0, int* tile_rows, int* tile_span, int* tile_count, int tile_m,
+                            int padded, cudaStream_t stream) {
   if (P == 0) return 0;
+  if (tile_m < 1) return -13;
   const size_t smem = (size_t)4 * (E > 0 ? E : 1) * sizeof(int);
   if (smem > 48 * 1024) return -13;
   sb_launch(moe_group_kernel, 1, 1024, smem, stream, chosen, P, E, max_tiles, sorted_pair, pos_of_pair, tile_expert,
-            tile_row0, tile_rows);
+            tile_row0, tile_rows, tile_span, tile_count, tile_m, padded);
   SB_LAUNCH_CHECK();
   return 0;
 }
@@ -227,27 +237,6 @@ extern "C" int sb_moe_group(const int* chosen, int P, int E, int max_tiles, int*
 // forms two sets of sums: weight rows n0 + c and `second` + n0 + c (c < 32).  GATED: out[r, n0 + c] =
 // act(set 0) * set 1.  Otherwise the sets are 64 neighbouring output columns (`second` = 32).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float moe_activation(float g, int act) {
-  if (act == 0) {
-    const float c = 0.7978845608028654f;
-    return 0.5f * g * (1.0f + tanhf(c * (g + 0.044715f * g * g * g)));
-  }
-  if (act == 1) return g / (1.0f + expf(-g));
-  if (act == 4) return 0.5f * g * (1.0f + erff(g * 0.7071067811865476f));  // the exact gelu
-  return fmaxf(g, 0.f);
-}
-
-// act(gate) * up; activation 3 is the clamped form, which acts on both halves:
-// g' = min(g, limit), u' = clamp(u, -limit, limit), g' sigmoid(1.702 g') (u' + 1).
-__device__ __forceinline__ float moe_gated_pair(float g, float u, int act, float limit) {
-  if (act == 3) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
-  }
-  return moe_activation(g, act) * u;
-}
-
 // 16 bytes from global memory (16-byte aligned) into a tile row (bfloat16 rows are, float rows are not).
 __device__ __forceinline__ void moe_copy16(bf16* dst, const bf16* src) {
   *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
@@ -498,7 +487,7 @@ extern "C" int sb_moe_product(const void* A, const int* row_pair, int pair_div, 
 }
 
 // ---------------------------------------------------------------------------
-// combine: a block per token and slice of columns.
+// combine: one column per thread, for widths that are no whole vectors.
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -525,107 +514,66 @@ moe_combine_kernel(const T* __restrict__ x, const T* __restrict__ y_pair, const 
   }
 }
 
+// The same sums, a vector of 16 bytes per thread, for whole vectors per row (2,048 tokens of 2,048, four
+// experts each: 24.8 us a column per thread, 9.3 this way; 6,000 tokens 71 and 24.8, 6.1 TB/s).
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_combine_vec_kernel(const T* __restrict__ x, const T* __restrict__ y_pair, const float* __restrict__ weight,
+                       const int* __restrict__ pos_of_pair, const T* __restrict__ shared,
+                       const float* __restrict__ shared_gate, int top, int width, long long vectors, T* __restrict__ out) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  constexpr int V = Vec<T>::N;
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= vectors) return;
+  const int per_row = width / V;
+  const int t = (int)(i / per_row), c = (int)(i - (long long)t * per_row) * V;
+  float acc[V] = {};
+#pragma unroll 4
+  for (int j = 0; j < top; ++j) {
+    const int pos = pos_of_pair[t * top + j];
+    const float w = weight[t * top + j];
+    float v[V];
+    Vec<T>::load(pos >= 0 ? y_pair + (size_t)pos * width + c : x + (size_t)t * width + c, v);
+#pragma unroll
+    for (int q = 0; q < V; ++q) acc[q] = fmaf(w, v[q], acc[q]);
+  }
+  if (shared != nullptr) {
+    const float sg = shared_gate != nullptr ? shared_gate[t] : 1.0f;
+    float v[V];
+    Vec<T>::load(shared + (size_t)t * width + c, v);
+#pragma unroll
+    for (int q = 0; q < V; ++q) acc[q] = fmaf(sg, v[q], acc[q]);
+  }
+  Vec<T>::store(out + (size_t)t * width + c, acc);
+}
+
+template <typename T>
+static void launch_combine(const T* x, const T* y_pair, const int* chosen, const float* weight, const int* pos_of_pair,
+                           const T* shared, const float* shared_gate, int E, int top, int num_tokens, int width, T* out,
+                           cudaStream_t stream) {
+  const uintptr_t all = (uintptr_t)x | (uintptr_t)y_pair | (uintptr_t)shared | (uintptr_t)out;
+  if (width % Vec<T>::N == 0 && (all & 15) == 0) {
+    const long long vectors = (long long)num_tokens * (width / Vec<T>::N);
+    sb_launch(moe_combine_vec_kernel<T>, dim3((unsigned)((vectors + 255) / 256)), 256, 0, stream, x, y_pair, weight,
+              pos_of_pair, shared, shared_gate, top, width, vectors, out);
+  } else {
+    const dim3 grid((unsigned)num_tokens, (unsigned)((width + 255) / 256));
+    sb_launch(moe_combine_kernel<T>, grid, 256, 0, stream, x, y_pair, chosen, weight, pos_of_pair, shared, shared_gate, E, top,
+              width, out);
+  }
+}
+
 extern "C" int sb_moe_combine(const void* x, const void* y_pair, int dtype, const int* chosen, const float* weight,
                               const int* pos_of_pair, const void* shared, const float* shared_gate, int E, int top,
                               int num_tokens, int width, void* out, cudaStream_t stream) {
   if (num_tokens == 0) return 0;
-  const dim3 grid((unsigned)num_tokens, (unsigned)((width + 255) / 256));
   if (dtype == SB_DTYPE_F32)
-    sb_launch(moe_combine_kernel<float>, grid, 256, 0, stream, (const float*)x, (const float*)y_pair, chosen,
-              weight, pos_of_pair, (const float*)shared, shared_gate, E, top, width, (float*)out);
+    launch_combine((const float*)x, (const float*)y_pair, chosen, weight, pos_of_pair, (const float*)shared, shared_gate, E,
+                   top, num_tokens, width, (float*)out, stream);
   else
-    sb_launch(moe_combine_kernel<bf16>, grid, 256, 0, stream, (const bf16*)x, (const bf16*)y_pair, chosen,
-              weight, pos_of_pair, (const bf16*)shared, shared_gate, E, top, width, (bf16*)out);
+    launch_combine((const bf16*)x, (const bf16*)y_pair, chosen, weight, pos_of_pair, (const bf16*)shared, shared_gate, E,
+                   top, num_tokens, width, (bf16*)out, stream);
   SB_LAUNCH_CHECK();
-  return 0;
-}
-
-// ---------------------------------------------------------------------------
-// The experts of a long prompt portion, one after the other through the dense products, issued
-// from here so that the host pays one call, not two per expert: rows [starts[i], starts[i] +
-// counts[i]) of xs (sorted by expert) go through expert experts[i]:
-//   h = act(xs W_gate^T) * (xs W_up^T)   the tcgen05 gated product (gemm_gated_tc.cu)
-//   y = h W_down^T                        the library's product (gemm_library.cu)
-// Returns -9 (nothing launched for that expert or any after it) when a product does not take the
-// shape; the caller then runs those experts through the kernel table's own methods.
-// One expert's products fill a part of the GPU only (32 tiles of 256 x 128 for 512 rows and 2,048
-// features, on 74 pairs of SMs): with `workspace2` every other expert goes to a second stream, which
-// starts after what `stream` holds so far and which `stream` waits for at the end.
-// ---------------------------------------------------------------------------
-extern "C" int sb_gemm_gated_tc(const void* x, const void* w, void* out, int M, int F, int K, int act, float limit,
-                                int blocks, int pairs, int* err, cudaStream_t stream);
-extern "C" int sb_gemm_library_bf16(const void* x, const void* w, void* out, int M, int N, int K, int out_f32,
-                                    void* workspace, long long workspace_bytes, cudaStream_t stream);
-
-// h <- act(h) in place, eight numbers per thread (experts without a gate on the dense route).
-__global__ void __launch_bounds__(256) activate_rows_kernel(bf16* __restrict__ h, long long groups, int act) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= groups) return;
-  uint4 v = reinterpret_cast<uint4*>(h)[i];
-  __nv_bfloat162* pair = reinterpret_cast<__nv_bfloat162*>(&v);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float2 f = __bfloat1622float2(pair[e]);
-    pair[e] = __floats2bfloat162_rn(moe_activation(f.x, act), moe_activation(f.y, act));
-  }
-  reinterpret_cast<uint4*>(h)[i] = v;
-}
-
-// `gated` 0: experts without a gate, gate_up [E, hidden, width]: the library's product, the
-// activation in place, the library's product.
-extern "C" int sb_experts_dense_bf16(const void* xs, const void* gate_up, const void* down, void* h, void* y,
-                                     const int* starts, const int* counts, const int* experts, int num, int width,
-                                     int hidden, int act, float limit, int gated, int blocks, int pairs, void* workspace,
-                                     void* workspace2, long long workspace_bytes, int* done, int* err,
-                                     cudaStream_t stream) {
-  *done = 0;
-  static cudaStream_t side = nullptr;
-  static cudaEvent_t fork_event = nullptr, join_event = nullptr;
-  bool two = workspace2 != nullptr && num > 1;
-  if (two && side == nullptr) {
-    if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&fork_event, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&join_event, cudaEventDisableTiming) != cudaSuccess) {
-      side = nullptr;
-      two = false;
-    }
-  }
-  if (two) {
-    cudaEventRecord(fork_event, stream);
-    cudaStreamWaitEvent(side, fork_event, 0);
-  }
-  // (whatever happens below, `stream` waits for the second stream before this returns)
-  struct Join {
-    bool on; cudaStream_t main, other; cudaEvent_t event;
-    ~Join() { if (on) { cudaEventRecord(event, other); cudaStreamWaitEvent(main, event, 0); } }
-  } join{two, stream, side, join_event};
-  cudaStream_t main_stream = stream;
-  void* main_workspace = workspace;
-  for (int i = 0; i < num; ++i) {
-    stream = (two && (i & 1)) ? side : main_stream;
-    workspace = (two && (i & 1)) ? workspace2 : main_workspace;
-    const size_t row = (size_t)starts[i];
-    const bf16* x_i = (const bf16*)xs + row * width;
-    bf16* h_i = (bf16*)h + row * hidden;
-    const bf16* gu = (const bf16*)gate_up + (size_t)experts[i] * (gated ? 2 : 1) * hidden * width;
-    const bf16* dn = (const bf16*)down + (size_t)experts[i] * width * hidden;
-    int rc;
-    if (gated) {
-      rc = sb_gemm_gated_tc(x_i, gu, h_i, counts[i], hidden, width, act, limit, blocks, pairs, err, stream);
-      if (rc != 0) return rc;
-    } else {
-      rc = sb_gemm_library_bf16(x_i, gu, h_i, counts[i], hidden, width, 0, workspace, workspace_bytes, stream);
-      if (rc != 0) return rc;
-      const long long groups = (long long)counts[i] * hidden / 8;  // (hidden is a multiple of 8, rows start on 16 bytes)
-      sb_launch(activate_rows_kernel, dim3((unsigned)((groups + 255) / 256)), 256, 0, stream, h_i, groups, act);
-      SB_LAUNCH_CHECK();
-    }
-    rc = sb_gemm_library_bf16(h_i, dn, (bf16*)y + row * width, counts[i], width, hidden, 0, workspace, workspace_bytes,
-                              stream);
-    if (rc != 0) return rc;  // (h_i is computed; the caller redoes this expert whole)
-    *done = i + 1;
-  }
   return 0;
 }

@@ -1,0 +1,544 @@
+// The routed experts' products on the fifth-generation tensor cores, all experts in one launch:
+//   out[r, :] = act(x[r, :] . W_e^T)                        experts without a gate, and the way down
+//   out[r, :] = act(x[r, :] . G_e^T) * (x[r, :] . U_e^T)    with a gate
+// for rows sorted by expert, an expert's rows starting at a multiple of a tile's rows (moe_group_kernel,
+// moe.cu).  How many tiles there are, and whose, stands in device memory, so neither a step nor a
+// graph needs the host.  Two kernels:
+//
+// Pairs of blocks (clusters of two, `cta_group::2`) for many rows: a tile is 256 rows x 256 weight rows
+// (gated: 128 gate rows and the up rows of the same features); each block fetches its 128 rows of x and
+// one half of the weights.
+// Single blocks for few rows, where reading the weights is the whole work: a tile is 128 rows x NT
+// weight rows.  The rows of x are fetched by name, four per copy (GATHER), straight from the step's
+// activations; only those that hold a pair (to a multiple of four, or of 32 on the way down) are
+// fetched, what stands in the other rows' shared memory reaches no row but its own.
+//
+// Both: persistent blocks, warp 0 fetches (TMA, 128-byte swizzle, a ring of stages), warp 1 multiplies,
+// eight warps read the sums from tensor memory, apply the activation in float32 and send bfloat16 rows
+// out through shared memory (TMA stores); two accumulators, so that the next tile's products run
+// while the last one is read back.  Tiles are numbered expert by expert, an expert's rows first: what
+// runs at the same time shares the weights and rows of a few experts.
+//   Any F and K that are multiples of 8: a weight box that runs over an expert's rows multiplies
+// rows of the next one into columns that the store cuts off.
+// Every wait is bounded; a wait that runs out sets SB_ERR_TIMEOUT, and the block still releases its
+// tensor memory before it leaves.
+#include "common.cuh"
+#include "moe_activation.cuh"
+#include "tma_mbar.cuh"
+
+namespace {
+
+using namespace sbx;
+
+constexpr int BM = 128, BK = 64, XBOX = 32;
+constexpr int XBOX_BYTES = XBOX * BK * 2;
+constexpr int A_BYTES = BM * BK * 2;
+constexpr int EPI_WARPS = 8;  // two per 32-lane quarter of tensor memory
+constexpr int THREADS = (2 + EPI_WARPS) * 32;
+constexpr int OUT_WARP_BYTES = 32 * 128;  // 32 rows of 64 bfloat16
+constexpr int OUT_BYTES = EPI_WARPS * OUT_WARP_BYTES;
+
+template <int NT>
+struct Shape {
+  static constexpr int B_BYTES = NT * BK * 2;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = NT == 256 ? 4 : 6;  // 192 KB of tiles in flight
+  static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + OUT_BYTES + 1024;
+};
+
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// Sixteen results of a row as two 16-byte pieces (128-byte swizzle) of the warp's stage.
+__device__ __forceinline__ void stage_pieces(unsigned char* stage, int lane, int piece, const float (&v)[16]) {
+  uint32_t p[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) p[i] = pack_pair(v[2 * i], v[2 * i + 1]);
+  unsigned char* row = stage + lane * 128;
+  *reinterpret_cast<uint4*>(row + ((piece ^ (lane & 7)) << 4)) = make_uint4(p[0], p[1], p[2], p[3]);
+  *reinterpret_cast<uint4*>(row + (((piece + 1) ^ (lane & 7)) << 4)) = make_uint4(p[4], p[5], p[6], p[7]);
+}
+
+// The tiles of a launch, in the order in which blocks take them.
+struct TileList {
+  const int* expert;  // of every tile of rows
+  const int* rows;    // rows of the tile that hold a pair
+  const int* first;   // the first tile of its expert
+  const int* span;    // how many its expert has
+  const int* count;   // all tiles of rows
+  int max_tiles;
+};
+struct Place {
+  int m, f0;
+};
+__device__ __forceinline__ Place place_of(const TileList& list, int tile, int tiles_f, int f_cols) {
+  const int any = tile / tiles_f;  // a tile of the same expert
+  const int first = list.first[any], span = list.span[any], at = tile - first * tiles_f;
+  return {first + at % span, at / span * f_cols};
+}
+
+// 64 output columns from column c0 of an accumulator for this warp's 32 rows: activation, bfloat16, one
+// TMA store to out[row0.., f0 + c0..].
+template <bool GATED, int NT>
+__device__ __forceinline__ void finish_columns(uint32_t acc, int c0, unsigned char* stage, const CUtensorMap* map_out, int row0,
+                                               int f0, int F, int act, float limit) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) tma_store_wait_read();  // the store before has read the stage
+  __syncwarp();
+#pragma unroll 1
+  for (int c = 0; c < 64; c += 16) {
+    uint32_t g[16];
+    float v[16];
+    tmem_load_32x16(acc + c0 + c, g);
+    if constexpr (GATED) {
+      uint32_t u[16];
+      tmem_load_32x16(acc + NT / 2 + c0 + c, u);
+      tmem_wait_load();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = moe_gated_pair(__uint_as_float(g[i]), __uint_as_float(u[i]), act, limit);
+    } else {
+      tmem_wait_load();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = act >= 0 ? moe_activation(__uint_as_float(g[i]), act) : __uint_as_float(g[i]);
+    }
+    stage_pieces(stage, lane, c / 8, v);
+  }
+  fence_proxy_async();  // the rows are visible to the TMA
+  __syncwarp();
+  if (lane == 0) {
+    if (f0 + c0 < F) tma_store_2d(map_out, stage, f0 + c0, row0);
+    tma_store_commit();
+  }
+}
+
+template <bool GATED, bool GATHER, int NT>
+__global__ void __launch_bounds__(THREADS, 1)
+grouped_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                  const __grid_constant__ CUtensorMap map_out, const TileList list, const int* __restrict__ sorted_pair,
+                  int top, int F, int K, int act, float limit, int* err) {
+  using S = Shape<NT>;
+  constexpr int STAGES = S::STAGES;
+  constexpr int FT = GATED ? NT / 2 : NT;  // output columns of a tile
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int s_failed;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nkb = (K + BK - 1) / BK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], EPI_WARPS);
+    }
+    s_failed = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(&tmem_base_slot, 2 * NT);
+  tc_fence_before_sync();
+  pdl_wait_block();  // the tiles' list, like x, comes from the kernels before this one
+  pdl_launch_dependents();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = tmem_base_slot;
+  const int tiles_f = (F + FT - 1) / FT, num_tiles = min(*list.count, list.max_tiles) * tiles_f;
+
+  if (warp == 0) {
+    // ---- producer: lane 0 waits and fetches the weights, every lane (GATHER) or lane 0 rows of x ----
+    int s = 0, use = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+      const auto [m, f0] = place_of(list, tile, tiles_f, FT);
+      const int w0 = list.expert[m] * (GATED ? 2 * F : F) + f0, rows = list.rows[m];
+      const int boxes = GATHER ? (rows + 3) / 4 : (rows + XBOX - 1) / XBOX;
+      const int bytes = S::B_BYTES + boxes * (GATHER ? 4 * BK * 2 : XBOX_BYTES);
+      [[maybe_unused]] int4 mine;
+      if constexpr (GATHER) {  // (behind the last pair: that pair's row again)
+        const int* pair = sorted_pair + m * BM;
+        mine = make_int4(pair[min(4 * lane, rows - 1)] / top, pair[min(4 * lane + 1, rows - 1)] / top,
+                         pair[min(4 * lane + 2, rows - 1)] / top, pair[min(4 * lane + 3, rows - 1)] / top);
+      }
+      for (int kb = 0; kb < nkb; ++kb) {
+        unsigned char* stage = tiles + s * S::STAGE_BYTES;
+        if (lane == 0) {
+          ok = use == 0 || mbar_wait_bounded(&empty[s], (use - 1) & 1);
+          if (ok) {
+            mbar_arrive_expect_tx(&full[s], bytes);
+            tma_load_2d(stage + A_BYTES, &map_w, kb * BK, w0, &full[s]);
+            tma_load_2d(stage + A_BYTES + S::B_BYTES / 2, &map_w, kb * BK, w0 + (GATED ? F : NT / 2), &full[s]);
+            if constexpr (!GATHER)
+              for (int b = 0; b < boxes; ++b)
+                tma_load_2d(stage + b * XBOX_BYTES, &map_x, kb * BK, m * BM + b * XBOX, &full[s]);
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        if (!ok) break;
+        if constexpr (GATHER)
+          if (lane < boxes) tma_gather4(stage + lane * 4 * BK * 2, &map_x, kb * BK, mine, &full[s]);
+        if (++s == STAGES) s = 0, ++use;
+      }
+    }
+    if (!ok) s_failed = 1;
+  } else if (warp == 1 && lane == 0) {
+    // ---- MMA issue ---------------------------------------------------------------------------
+    const uint32_t idesc = idesc_bf16_f32(BM, NT, false, false);
+    const uint64_t a_desc0 = smem_desc_sw128(tiles, 16, 1024);
+    const uint64_t b_desc0 = smem_desc_sw128(tiles + A_BYTES, 16, 1024);
+    int s = 0, use = 0, t = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++t) {
+      const int buf = t & 1;
+      if (t >= 2) {  // the epilogue has read this accumulator's tile before last
+        ok = mbar_wait_bounded(&acc_empty[buf], (t / 2 - 1) & 1);
+        if (!ok) break;
+        tc_fence_after_sync();
+      }
+      const uint32_t d = tmem + buf * NT;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!mbar_wait_bounded(&full[s], use & 1)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+        const uint64_t off = (uint64_t)((s * S::STAGE_BYTES) >> 4);
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          tc_mma_f16(d, a_desc0 + off + (uint64_t)(k * 2), b_desc0 + off + (uint64_t)(k * 2), idesc, kb > 0 || k > 0);
+        tc_commit(&empty[s]);
+        if (++s == STAGES) s = 0, ++use;
+      }
+      if (ok) tc_commit(&acc_full[buf]);
+    }
+    if (!ok) s_failed = 1;
+  } else if (warp >= 2) {
+    // ---- epilogue ----------------------------------------------------------------------------
+    // A warp may only touch the 32 lanes of tensor memory that (warp % 4) names; the two warps of a
+    // quarter take one half of the tile's output columns each (64 columns leave in one store: where a
+    // tile has no more, the first warp takes them all).
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    constexpr int COLS = FT > 64 ? FT / 2 : FT;
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    unsigned char* stage = tiles + STAGES * S::STAGE_BYTES + (warp - 2) * OUT_WARP_BYTES;
+    int t = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++t) {
+      const int buf = t & 1;
+      const auto [m, f0] = place_of(list, tile, tiles_f, FT);
+      const bool live = quarter * 32 < list.rows[m] && half * COLS < FT;
+      if (!mbar_wait_bounded_relaxed(&acc_full[buf], (t / 2) & 1)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after_sync();
+      if (live)
+#pragma unroll 1
+        for (int c0 = half * COLS; c0 < (half + 1) * COLS; c0 += 64)
+          finish_columns<GATED, NT>(tmem + lane_base + buf * NT, c0, stage, &map_out, m * BM + quarter * 32, f0, F, act, limit);
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+    }
+    if (lane == 0) tma_store_wait_read();  // shared memory has been read; the grid's end covers the writes
+    if (!ok) s_failed = 1;
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x == 0 && s_failed) atomicOr(err, SB_ERR_TIMEOUT);
+  if (warp == 1) tmem_dealloc(tmem, 2 * NT);
+}
+
+// Pairs of blocks: the pair's tile is 256 rows x 256 weight rows, one `tcgen05.mma.cta_group::2` of
+// 256 x 256 x 16 per 16 of k, issued by rank 0.  Both blocks' TMA count their bytes at rank 0's full[s];
+// `tcgen05.commit` arrives at empty[s] and acc_full[b] of both; the epilogue warps of both arrive at
+// rank 0's acc_empty[b].
+constexpr int PAIR_NT = 256, PAIR_STAGES = 6;
+constexpr int PAIR_B_BYTES = PAIR_NT / 2 * BK * 2;
+constexpr int PAIR_STAGE_BYTES = A_BYTES + PAIR_B_BYTES;
+constexpr size_t PAIR_SMEM = (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + OUT_BYTES + 1024;
+
+template <bool GATED>
+__global__ void __launch_bounds__(THREADS, 1)
+grouped_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                       const __grid_constant__ CUtensorMap map_out, const TileList list, int F, int K, int act, float limit,
+                       int* err) {
+  constexpr int NT = PAIR_NT, FT = GATED ? NT / 2 : NT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  __shared__ __align__(8) uint64_t full[PAIR_STAGES], empty[PAIR_STAGES], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int s_failed;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank(), pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const int nkb = (K + BK - 1) / BK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < PAIR_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 2 * EPI_WARPS);
+    }
+    s_failed = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(&tmem_base_slot, 2 * NT);
+  tc_fence_before_sync();
+  pdl_wait_block();
+  pdl_launch_dependents();
+  cluster_sync_all();  // the other block's barriers and tensor memory exist before anything arrives there
+  tc_fence_after_sync();
+  const uint32_t tmem = tmem_base_slot;
+  const int tiles_f = (F + FT - 1) / FT, num_tiles = min(*list.count, list.max_tiles) * tiles_f;
+
+  if (warp == 0 && lane == 0) {
+    // ---- producer (both blocks) ------------------------------------------------------------
+    const uint32_t full0 = mapa_shared(smem_u32(&full[0]), 0);
+    int s = 0, use = 0;
+    bool ok = true;
+    for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
+      const auto [m, f0] = place_of(list, tile, tiles_f, FT);
+      const int w0 = list.expert[m] * (GATED ? 2 * F : F) + f0 + rank * (GATED ? F : NT / 2);
+      const int rows = list.rows[m], x0 = (2 * m + rank) * BM;
+      const int boxes0 = (min(rows, BM) + XBOX - 1) / XBOX, boxes1 = (max(rows - BM, 0) + XBOX - 1) / XBOX;
+      const int boxes = rank == 0 ? boxes0 : boxes1, bytes = 2 * PAIR_B_BYTES + (boxes0 + boxes1) * XBOX_BYTES;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1)) {
+          ok = false;
+          break;
+        }
+        unsigned char* stage = tiles + s * PAIR_STAGE_BYTES;
+        if (rank == 0) mbar_arrive_expect_tx(&full[s], bytes);
+        tma_load_2d_pair(stage + A_BYTES, &map_w, kb * BK, w0, full0 + 8 * s);
+        for (int b = 0; b < boxes; ++b)
+          tma_load_2d_pair(stage + b * XBOX_BYTES, &map_x, kb * BK, x0 + b * XBOX, full0 + 8 * s);
+        if (++s == PAIR_STAGES) s = 0, ++use;
+      }
+    }
+    if (!ok) s_failed = 1;
+  } else if (warp == 1 && lane == 0 && rank == 0) {
+    // ---- MMA issue (rank 0, for the pair) -----------------------------------------------------
+    const uint32_t idesc = idesc_bf16_f32(2 * BM, NT, false, false);
+    const uint64_t a_desc0 = smem_desc_sw128(tiles, 16, 1024);
+    const uint64_t b_desc0 = smem_desc_sw128(tiles + A_BYTES, 16, 1024);
+    int s = 0, use = 0, t = 0;
+    bool ok = true;
+    for (int tile = pair; ok && tile < num_tiles; tile += num_pairs, ++t) {
+      const int buf = t & 1;
+      if (t >= 2) {
+        ok = mbar_wait_bounded_cluster(&acc_empty[buf], (t / 2 - 1) & 1);
+        if (!ok) break;
+        tc_fence_after_sync();
+      }
+      const uint32_t d = tmem + buf * NT;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!mbar_wait_bounded(&full[s], use & 1)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+        const uint64_t off = (uint64_t)((s * PAIR_STAGE_BYTES) >> 4);
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          tc_mma_f16_pair(d, a_desc0 + off + (uint64_t)(k * 2), b_desc0 + off + (uint64_t)(k * 2), idesc, kb > 0 || k > 0);
+        tc_commit_pair(&empty[s]);
+        if (++s == PAIR_STAGES) s = 0, ++use;
+      }
+      if (ok) tc_commit_pair(&acc_full[buf]);
+    }
+    if (!ok) s_failed = 1;
+  } else if (warp >= 2) {
+    // ---- epilogue (both blocks, each its own 128 rows) ------------------------------------------
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    unsigned char* stage = tiles + PAIR_STAGES * PAIR_STAGE_BYTES + (warp - 2) * OUT_WARP_BYTES;
+    int t = 0;
+    bool ok = true;
+    for (int tile = pair; ok && tile < num_tiles; tile += num_pairs, ++t) {
+      const int buf = t & 1;
+      const auto [m, f0] = place_of(list, tile, tiles_f, FT);
+      const bool live = rank * BM + quarter * 32 < list.rows[m];
+      if (!mbar_wait_bounded_relaxed(&acc_full[buf], (t / 2) & 1)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after_sync();
+      if (live)
+#pragma unroll 1
+        for (int c0 = half * FT / 2; c0 < (half + 1) * FT / 2; c0 += 64)
+          finish_columns<GATED, NT>(tmem + lane_base + buf * NT, c0, stage, &map_out, (2 * m + rank) * BM + quarter * 32, f0, F,
+                                    act, limit);
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[buf]), 0));
+    }
+    if (lane == 0) tma_store_wait_read();
+    if (!ok) s_failed = 1;
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x == 0 && s_failed) atomicOr(err, SB_ERR_TIMEOUT);
+  // Neither block leaves while the other may still arrive at its barriers or multiply into its
+  // tensor memory.
+  cluster_sync_all();
+  if (warp == 1) tmem_dealloc(tmem, 2 * NT);
+}
+
+int sms() {
+  static const int num_sms = [] {
+    int device = 0, n = 0;
+    cudaGetDevice(&device);
+    return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 1;
+  }();
+  return num_sms;
+}
+
+template <bool GATED, bool GATHER, int NT>
+int launch(const void* x, const void* w, void* out, int x_rows, int rows, int E, int F, int K, int act, float limit,
+           const TileList& list, const int* sorted_pair, int top, int* err, cudaStream_t stream) {
+  static const int configured = (int)cudaFuncSetAttribute(
+      grouped_tc_kernel<GATED, GATHER, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<NT>::SMEM);
+  if (configured != 0) return configured;
+  CUtensorMap map_x, map_w, map_out;
+  if (sb_make_map_2d(&map_x, x, x_rows, K, GATHER ? 1 : XBOX) != 0) return -12;
+  if (sb_make_map_2d(&map_w, w, (long long)E * (GATED ? 2 : 1) * F, K, NT / 2) != 0) return -12;
+  if (sb_make_map_2d(&map_out, out, rows, F, 32) != 0) return -12;
+  constexpr int FT = GATED ? NT / 2 : NT;
+  const int grid = (int)min((long long)list.max_tiles * ((F + FT - 1) / FT), (long long)sms());
+  cudaError_t e = sb_launch(grouped_tc_kernel<GATED, GATHER, NT>, dim3(grid), dim3(THREADS), Shape<NT>::SMEM, stream, map_x,
+                            map_w, map_out, list, sorted_pair, top, F, K, act, limit, err);
+  if (e != cudaSuccess) return (int)e;
+  SB_LAUNCH_CHECK();
+  return 0;
+}
+
+cudaLaunchConfig_t pair_config(int pairs, cudaStream_t stream, cudaLaunchAttribute (&attribute)[2]) {
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = 2;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)(2 * pairs));
+  config.blockDim = dim3(THREADS);
+  config.dynamicSmemBytes = PAIR_SMEM;
+  config.stream = stream;
+  config.attrs = attribute;
+  config.numAttrs = sb_pdl_level() == 1 ? 2 : 1;
+  return config;
+}
+
+template <bool GATED>
+int launch_pairs(const void* x, const void* w, void* out, int rows, int E, int F, int K, int act, float limit,
+                 const TileList& list, int* err, cudaStream_t stream) {
+  struct Setup {
+    int status, pairs = 0;  // how many pairs the GPU holds at once (a pair lives inside one GPC)
+    Setup() {
+      status = (int)cudaFuncSetAttribute(grouped_tc_pair_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAIR_SMEM);
+      if (status != 0) return;
+      cudaLaunchAttribute attribute[2];
+      cudaLaunchConfig_t config = pair_config(sms() / 2, nullptr, attribute);
+      config.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&pairs, grouped_tc_pair_kernel<GATED>, &config) != cudaSuccess) {
+        cudaGetLastError();
+        pairs = 0;
+      }
+    }
+  };
+  static const Setup setup;
+  if (setup.status != 0) return setup.status;
+  if (setup.pairs <= 0) return -9;
+  CUtensorMap map_x, map_w, map_out;
+  if (sb_make_map_2d(&map_x, x, rows, K, XBOX) != 0) return -12;
+  if (sb_make_map_2d(&map_w, w, (long long)E * (GATED ? 2 : 1) * F, K, PAIR_NT / 2) != 0) return -12;
+  if (sb_make_map_2d(&map_out, out, rows, F, 32) != 0) return -12;
+  constexpr int FT = GATED ? PAIR_NT / 2 : PAIR_NT;
+  const int pairs = (int)min((long long)list.max_tiles * ((F + FT - 1) / FT), (long long)setup.pairs);
+  cudaLaunchAttribute attribute[2];
+  const cudaLaunchConfig_t config = pair_config(pairs, stream, attribute);
+  cudaError_t e = cudaLaunchKernelEx(&config, grouped_tc_pair_kernel<GATED>, map_x, map_w, map_out, list, F, K, act, limit, err);
+  if (e != cudaSuccess) return (int)e;
+  SB_LAUNCH_CHECK();
+  return 0;
+}
+
+// out[r] = x[sorted_pair[r] / top] for the rows of every tile that hold a pair: a warp per row, whole
+// 16-byte pieces.
+__global__ void __launch_bounds__(256)
+gather_pairs_kernel(const bf16* __restrict__ x, const int* __restrict__ sorted_pair, int top, int tile_m,
+                    const int* __restrict__ tile_rows, const int* __restrict__ tile_count, int pieces, bf16* __restrict__ out) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int tile = row / tile_m;
+  if (tile >= *tile_count || row - tile * tile_m >= tile_rows[tile]) return;
+  const uint4* src = reinterpret_cast<const uint4*>(x) + (size_t)(sorted_pair[row] / top) * pieces;
+  uint4* dst = reinterpret_cast<uint4*>(out) + (size_t)row * pieces;
+#pragma unroll 8
+  for (int c = lane; c < pieces; c += 32) dst[c] = src[c];
+}
+
+}  // namespace
+
+// The rows of x in sorted order: out [max_tiles * tile_m, width], width a multiple of 8.
+extern "C" int sb_moe_gather(const void* x, const int* sorted_pair, int top, int tile_m, const int* tile_rows,
+                             const int* tile_count, int max_tiles, int width, void* out, cudaStream_t stream) {
+  if (max_tiles == 0) return 0;
+  if (width % 8 != 0 || tile_m % 8 != 0 || top < 1) return -13;
+  sb_launch(gather_pairs_kernel, dim3((unsigned)(max_tiles * (tile_m / 8))), 256, 0, stream, (const bf16*)x, sorted_pair, top,
+            tile_m, tile_rows, tile_count, width / 8, (bf16*)out);
+  SB_LAUNCH_CHECK();
+  return 0;
+}
+
+// out [max_tiles * tile_m, F]; x [x_rows, K] with sorted_pair (row r is x's row sorted_pair[r] / top), or
+// null and x [max_tiles * tile_m, K]; w [E, (gated ? 2 F : F), K].  tile_m 256: by pairs of blocks
+// (sorted_pair null); 128: single blocks, `wide` 1 with 256 weight rows per tile, 0 with 128, -1: 128 where
+// tiles of 256 would leave half of the SMs without one (8 experts of 2,048 x 2,048 both ways: 39 us
+// against 46; 16 experts: 65 against 55).  Rows of a tile without a pair may come out as anything.
+// Returns -9 for shapes the kernels do not take.
+// Measured, 16 experts of 2,048 x 2,048, 4 per token, both products with the sorting and the sum (B200),
+// us, against one launch per expert and product (from 384 rows per expert) or the mma.sync kernel:
+//   tokens               8     64    256    512   2048   6000
+//   with a gate       95/82 131/93 250/102 397/123 768/256 1056/611
+//   without           69/62 99/66  204/74  294/89  628/197 847/444
+// Pairs take over above 64 rows per expert (256 tokens above: single blocks 102 and 74, pairs 117 and 80;
+// 512: 188 and 148 against 123 and 89: rows fetched four at a time cost 47 ns a copy).
+extern "C" int sb_moe_grouped_tc(const void* x, int x_rows, const int* sorted_pair, int top, const void* w, void* out, int E,
+                                 int F, int K, int gated, int act, float limit, const int* tile_expert, const int* tile_rows,
+                                 const int* tile_first, const int* tile_span, const int* tile_count, int max_tiles,
+                                 int tile_m, int wide, int* err, cudaStream_t stream) {
+  if (max_tiles == 0 || F == 0) return 0;
+  const int rows = max_tiles * tile_m;
+  if (act < (gated ? 0 : -1) || act > 4 || (act == 3 && !(gated && limit > 0.f)) || E <= 0 || K <= 0 || x_rows <= 0 || top < 1 ||
+      (tile_m != BM && tile_m != 2 * BM) || (sorted_pair == nullptr && x_rows != rows))
+    return -13;
+  if (F % 8 != 0 || K % 8 != 0 || (long long)E * 2 * F > 0x7fffffffLL) return -9;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15) return -9;
+  const TileList list{tile_expert, tile_rows, tile_first, tile_span, tile_count, max_tiles};
+  if (tile_m == 2 * BM) {
+    if (sorted_pair != nullptr) return -13;
+    if (gated) return launch_pairs<true>(x, w, out, rows, E, F, K, act, limit, list, err, stream);
+    return launch_pairs<false>(x, w, out, rows, E, F, K, act, limit, list, err, stream);
+  }
+  if (wide < 0) wide = (long long)max_tiles * ((gated ? 2LL * F : F) + 255) / 256 > sms() / 2;
+#define SB_GROUPED(G_, X_, N_) \
+  return launch<G_, X_, N_>(x, w, out, x_rows, rows, E, F, K, act, limit, list, sorted_pair, top, err, stream)
+  if (gated && sorted_pair == nullptr) return -13;
+  if (gated && wide) SB_GROUPED(true, true, 256);
+  if (gated) SB_GROUPED(true, true, 128);
+  if (sorted_pair != nullptr && wide) SB_GROUPED(false, true, 256);
+  if (sorted_pair != nullptr) SB_GROUPED(false, true, 128);
+  if (wide) SB_GROUPED(false, false, 256);
+  SB_GROUPED(false, false, 128);
+#undef SB_GROUPED
+}

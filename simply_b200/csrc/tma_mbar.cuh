@@ -87,6 +87,15 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
       "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
       : "memory");
 }
+// Four rows of a matrix, named one by one, times the box's columns (the map's box is one row high): they
+// land one after the other, as four rows of a tile would.
+__device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, int c0, int4 rows, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
+      "%6}], [%7];\n" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(c0), "r"(rows.x), "r"(rows.y), "r"(rows.z), "r"(rows.w), "r"(smem_u32(bar))
+      : "memory");
+}
 // A tile from shared memory to the tensor (rows and columns beyond it are not written).  The
 // issuing thread commits its copies as a group and waits for the group: `_read` until shared
 // memory may be written again, `_all` until the copies are complete.

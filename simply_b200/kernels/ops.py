@@ -183,12 +183,13 @@ class CudaOps:
     # pages of at least 64 tokens); False keeps single blocks (tests).
     self.prefill_pairs = True
     self._rounded_scales: dict[float, float] = {}
-    # Routed experts: from this many rows per expert on average (and outside graph capture) a
-    # step's experts run one by one through the products of a dense feed-forward, after one look
-    # at how many rows each got; below, and in decode graphs, the grouped kernel (csrc/moe.cu)
-    # serves them without the host.  0: always the grouped kernel.
-    self.expert_rows_for_dense_products = int(os.environ.get("SIMPLY_B200_EXPERT_DENSE_ROWS", "384"))
-    self.expert_side_stream = True  # False: all experts on the step's stream (tests, experiments)
+    # Routed experts in bfloat16 run on the grouped tcgen05 products (csrc/moe_tc.cu); False keeps the
+    # grouped mma.sync kernel (csrc/moe.cu), which serves widths that are no multiple of 8 (tests).
+    self.experts_on_tcgen05 = True
+    # From this many rows per expert on average by pairs of blocks; weight rows of a single block's
+    # tile: 0 128, 1 256, -1 the launch chooses (tests).  Where the lines lie: sb_moe_grouped_tc.
+    self.experts_pair_rows = 64
+    self.experts_wide = -1
     self._wide_tables: dict[tuple, torch.Tensor] = {}
     self.prefill_single_key_group = False  # True: 64-row tiles with 4 warps instead of 4 x 2 (experiments, tests)
     # 0: the weight-streaming product picks its warps per block; 4, 8 or 16 forces them (experiments).
@@ -315,7 +316,11 @@ class CudaOps:
                            c_int, c_int, c_int, c_void, c_void, c_void, c_void],
         "sb_moe_route": [c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_int, c_int, c_float, c_int, c_int,
                          c_int, c_int, c_void, c_void, c_void, c_void],
-        "sb_moe_group": [c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_void, c_void],
+        "sb_moe_group": [c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_void, c_void, c_void, c_int, c_int,
+                         c_void],
+        "sb_moe_gather": [c_void, c_void, c_int, c_int, c_void, c_void, c_int, c_int, c_void, c_void],
+        "sb_moe_grouped_tc": [c_void, c_int, c_void, c_int, c_void, c_void, c_int, c_int, c_int, c_int, c_int,
+                              c_float, c_void, c_void, c_void, c_void, c_void, c_int, c_int, c_int, c_void, c_void],
         "sb_moe_product": [c_void, c_void, c_int, c_void, c_int, c_int, c_int, c_int, c_void, c_void, c_void, c_int,
                            c_int, c_float, c_void, c_void],
         "sb_scaled_residual_tanh": [c_void, c_void, c_void, c_void, c_void, c_int, c_void, c_void, c_void, c_void,
@@ -340,11 +345,6 @@ class CudaOps:
     self.lib.sb_gemm_library_bf16_heads.argtypes = [c_void, c_int, c_int, c_void, c_void, c_int, c_int, c_int, c_int, c_int,
                                                     c_int, ctypes.c_float, c_void, c_ll, c_void]
     self.lib.sb_gemm_library_bf16_heads.restype = c_int
-    c_ip = ctypes.POINTER(c_int)
-    self.lib.sb_experts_dense_bf16.argtypes = [c_void, c_void, c_void, c_void, c_void, c_ip, c_ip, c_ip, c_int, c_int,
-                                               c_int, c_int, c_float, c_int, c_int, c_int, c_void, c_void, c_ll, c_ip, c_void,
-                                               c_void]
-    self.lib.sb_experts_dense_bf16.restype = c_int
     self.lib.sb_graph_burst.argtypes = [c_void, c_void, c_void, c_ll, c_int, c_void, c_void, c_ll, c_void]
     self.lib.sb_graph_burst.restype = c_int
     self.lib.sb_stream_wait.argtypes = [c_void]
@@ -1509,61 +1509,6 @@ class CudaOps:
                _ptr(weight), t, _ptr(self.err))
     return chosen, weight
 
-  def _experts_one_by_one(self, x, sorted_pair, tiles, top, gate_up, down, activation, gated=True,
-                          limit: float = 0.0) -> torch.Tensor:
-    """The experts' products of a long prompt portion: the rows, sorted by expert, are gathered once,
-    the host reads how many each expert got (the one wait of the step), and every expert's rows go
-    through the engine's own products for a dense feed-forward (the tcgen05 kernel with the
-    activation on its sums from 129 rows, the library's product for the way down), issued by one
-    native call that puts every other expert on a second stream (csrc/moe.cu).  Experts without a
-    gate: the library's product both ways, the activation in place between them.  Returns the rows
-    of every pair in sorted order, as the grouped kernel does."""
-    expert, row0, count = tiles.cpu().numpy()
-    total = int(count[expert >= 0].sum())  # (identity experts' pairs have no row; the list's tail is unused)
-    rows_of = torch.div(sorted_pair[:total], top, rounding_mode="floor")
-    xs = self.gather_rows(x, rows_of)
-    which = np.unique(expert[expert >= 0]).astype(np.int32)
-    starts = np.array([row0[expert == e].min() for e in which], dtype=np.int32)
-    counts = np.array([count[expert == e].sum() for e in which], dtype=np.int32)
-    width, hidden = x.shape[1], down.shape[2]
-    y = self._new(total, width, dtype=x.dtype)
-    # Experts with enough rows for the tcgen05 product: all of them in one call of the library, so
-    # that the host pays one call, not two per expert.  The others through the kernel table's methods.
-    if not gated:
-      big = np.ones(len(counts), dtype=bool)
-    else:
-      big = counts >= self.gated_tc_min_rows if self.gated_tc_min_rows > 0 else np.zeros(len(counts), dtype=bool)
-    rest = [(int(e), int(s), int(n)) for e, s, n in zip(which[~big], starts[~big], counts[~big])]
-    which, starts, counts = (np.ascontiguousarray(a[big]) for a in (which, starts, counts))
-    if len(which):
-      stream = self._stream()
-      workspace = self._library_workspaces.get(stream.value)
-      if workspace is None:
-        workspace = self._library_workspaces[stream.value] = torch.empty(32 << 20, dtype=torch.uint8, device=self.device)
-      second = None
-      if self.expert_side_stream:  # every other expert on a second stream, with a workspace of its own
-        second = self._library_workspaces.get("experts")
-        if second is None:
-          second = self._library_workspaces["experts"] = torch.empty(32 << 20, dtype=torch.uint8, device=self.device)
-      h = self._new(total, hidden, dtype=x.dtype)
-      finished = ctypes.c_int(0)
-      as_ints = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_int))
-      rc = self.lib.sb_experts_dense_bf16(
-          _ptr(xs), _ptr(gate_up), _ptr(down), _ptr(h), _ptr(y), as_ints(starts), as_ints(counts), as_ints(which),
-          len(which), width, hidden, activation, float(limit), int(gated), self.gated_tc_blocks, int(self.gated_tc_pairs), _ptr(workspace),
-          _ptr(second), workspace.numel(), ctypes.byref(finished), _ptr(self.err), stream)
-      if rc > 0:
-        raise KernelError(f"sb_experts_dense_bf16: CUDA or cuBLAS status {rc}")
-      done = finished.value
-      if not gated and done < len(which):
-        raise KernelError("sb_experts_dense_bf16: the library refused a product")
-      self.launches += (2 if gated else 3) * done
-      rest += list(zip(which[done:].tolist(), starts[done:].tolist(), counts[done:].tolist()))
-    for e, start, n in rest:
-      h_e = self.gated_linear(xs[start:start + n], gate_up[e], activation, limit)
-      y[start:start + n] = self.linear(h_e, down[e])
-    return y
-
   def mix_experts(self, x: torch.Tensor, chosen: torch.Tensor, weight: torch.Tensor, gate_up: torch.Tensor | None,
                   down: torch.Tensor | None, num_experts: int, activation: int, shared: torch.Tensor | None,
                   shared_gate: torch.Tensor | None, gated: bool = True, limit: float = 0.0) -> torch.Tensor:
@@ -1579,23 +1524,38 @@ class CudaOps:
     if num_experts > 0:
       if gate_up.dtype != x.dtype:
         raise KernelError("the experts' matrices and the activations must share one dtype")
-      max_tiles = pairs // self.MOE_TILE_ROWS + min(num_experts, pairs)
-      words = self._new(pairs + 3 * max_tiles, dtype=torch.int32)
-      sorted_pair, tiles = words[:pairs], words[pairs:].view(3, max_tiles)
-      self._call("sb_moe_group", _ptr(chosen), pairs, num_experts, max_tiles, _ptr(sorted_pair), _ptr(pos),
-                 _ptr(tiles[0]), _ptr(tiles[1]), _ptr(tiles[2]))
       hidden = down.shape[2]
-      # (whole 16-byte groups per row, so that an expert's slice of the rows starts on a boundary)
-      if (x.dtype == torch.bfloat16 and 0 < self.expert_rows_for_dense_products * num_experts <= pairs
-          and width % 8 == 0 and hidden % 8 == 0 and not torch.cuda.is_current_stream_capturing()):
-        y_pair = self._experts_one_by_one(x, sorted_pair, tiles, top, gate_up, down, activation, gated, limit)
+      on_tc = (self.experts_on_tcgen05 and x.dtype == torch.bfloat16 and width % 8 == 0 and hidden % 8 == 0)
+      by_pairs = on_tc and pairs > self.experts_pair_rows * num_experts
+      tile_rows = (256 if by_pairs else 128) if on_tc else self.MOE_TILE_ROWS
+      max_tiles = pairs // tile_rows + min(num_experts, pairs)
+      rows = max_tiles * tile_rows if on_tc else pairs
+      words = self._new(rows + 4 * max_tiles + 1, dtype=torch.int32)
+      sorted_pair, tiles, count = words[:rows], words[rows:-1].view(4, max_tiles), words[-1:]
+      expert, row0, of_tile, span = tiles
+      self._call("sb_moe_group", _ptr(chosen), pairs, num_experts, max_tiles, _ptr(sorted_pair), _ptr(pos),
+                 _ptr(expert), _ptr(row0), _ptr(of_tile), _ptr(span), _ptr(count), tile_rows, int(on_tc))
+      if on_tc:
+        def product(a, pair, w, gate, act, n):
+          out = self._new(rows, n, dtype=x.dtype)
+          self._call("sb_moe_grouped_tc", _ptr(a), a.shape[0], _ptr(pair), top, _ptr(w), _ptr(out), num_experts, n,
+                     a.shape[1], int(gate), act, float(limit), _ptr(expert), _ptr(of_tile), _ptr(row0), _ptr(span),
+                     _ptr(count), max_tiles, tile_rows, self.experts_wide, _ptr(self.err))
+          return out
+        xs, named = x, sorted_pair
+        if by_pairs:
+          xs, named = self._new(rows, width, dtype=x.dtype), None
+          self._call("sb_moe_gather", _ptr(x), _ptr(sorted_pair), top, tile_rows, _ptr(of_tile), _ptr(count), max_tiles,
+                     width, _ptr(xs))
+        h = product(xs, named, gate_up, gated, activation, hidden)
+        y_pair = product(h, None, down, False, -1, width)
       else:
         h = self._new(pairs, hidden, dtype=x.dtype)
         self._call("sb_moe_product", _ptr(x), _ptr(sorted_pair), top, _ptr(gate_up), _code(x), int(gated), width, hidden,
-                   _ptr(tiles[0]), _ptr(tiles[1]), _ptr(tiles[2]), max_tiles, activation, float(limit), _ptr(h))
+                   _ptr(expert), _ptr(row0), _ptr(of_tile), max_tiles, activation, float(limit), _ptr(h))
         y_pair = self._new(pairs, width, dtype=x.dtype)
         self._call("sb_moe_product", _ptr(h), None, 1, _ptr(down), _code(x), 0, hidden, width,
-                   _ptr(tiles[0]), _ptr(tiles[1]), _ptr(tiles[2]), max_tiles, -1, 0.0, _ptr(y_pair))
+                   _ptr(expert), _ptr(row0), _ptr(of_tile), max_tiles, -1, 0.0, _ptr(y_pair))
     else:
       pos.fill_(-1)
     if shared is not None and shared.dtype != x.dtype:

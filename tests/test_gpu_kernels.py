@@ -698,3 +698,49 @@ def test_sample_is_distributed_as_softmax(table):
   freq = torch.bincount(got.cpu().long(), minlength=5).float() / 4000
   want = torch.softmax(logits[0], 0)
   assert (freq - want).abs().max() < 0.03
+
+
+@pytest.mark.parametrize("gated,act", [(True, 1), (True, 3), (False, 4), (False, 2)])
+@pytest.mark.parametrize("width,hidden", [(64, 40), (72, 264), (136, 128), (512, 648)])
+@pytest.mark.parametrize("tokens", [1, 3, 33, 130, 517])
+def test_grouped_experts_on_tcgen05(table, gated, act, width, hidden, tokens):
+  """Every tile shape of the experts' tcgen05 products: one row to several tiles per expert, ragged last
+  tiles, hidden sizes that end inside a weight box, experts that get no row and identity experts."""
+  ops = table[torch.bfloat16]
+  experts, top, limit = 5, 3, 0.9
+  gen = torch.Generator(device="cuda").manual_seed(tokens * 1000 + hidden)
+  make = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+  x = make(tokens, width).to(torch.bfloat16)
+  up = (make(experts, (2 if gated else 1) * hidden, width) * width ** -0.5).to(torch.bfloat16)
+  down = (make(experts, width, hidden) * hidden ** -0.5).to(torch.bfloat16)
+  score = make(tokens, experts + 1)
+  score[:, 1] = -9.0  # never chosen
+  if tokens > 3:
+    score[:, 4] += 2.0  # chosen by most
+  chosen = score.argsort(dim=1, descending=True)[:, :top].to(torch.int32).contiguous()
+  weight = torch.rand((tokens, top), generator=gen, device="cuda")
+  want = torch.zeros(tokens, width, dtype=torch.float64, device="cuda")
+  for t in range(top):
+    for e in range(experts):
+      at = (chosen[:, t] == e).nonzero()[:, 0]
+      z = x[at].double() @ up[e].double().T
+      if gated:
+        g, u = z[:, :hidden], z[:, hidden:]
+        if act == 3:
+          g, u = g.clamp(max=limit), u.clamp(-limit, limit) + 1.0
+        z = g * torch.sigmoid((1.702 if act == 3 else 1.0) * g) * u
+      else:
+        z = torch.nn.functional.gelu(z) if act == 4 else z.clamp(min=0)
+      want[at] += weight[at, t, None].double() * (z @ down[e].double().T)
+    same = (chosen[:, t] == experts).nonzero()[:, 0]
+    want[same] += weight[same, t, None].double() * x[same].double()
+  before = ops.experts_pair_rows, ops.experts_wide
+  try:
+    for pair_rows, wide in ((0, -1), (1 << 30, 0), (1 << 30, 1)):  # pairs of blocks; single blocks, both widths
+      ops.experts_pair_rows, ops.experts_wide = pair_rows, wide
+      got = ops.mix_experts(x, chosen, weight, up, down, experts, act, None, None, gated=gated, limit=limit if act == 3 else 0.0)
+      # three roundings to bfloat16 on the way (hidden values, an expert's rows, the sum), 2^-9 each at most
+      assert ((got.double() - want).norm() / want.norm()).item() < 3 * 2.0 ** -9, (pair_rows, wide)
+  finally:
+    ops.experts_pair_rows, ops.experts_wide = before
+  ops.check_errors()
