@@ -1,0 +1,574 @@
+// Long walks through recurrent states, a chunk of Q tokens at a time as products of small matrices.
+//
+// A step of one token is a row of products with the state and a rank-one update of it: every
+// multiply-add fetches its operand from shared memory and every output is a sum over lanes.  Taken
+// Q tokens together the same sums are
+//     out[Q x dv]  = rs . (X1[Q x N] S) + A[Q x Q] V         S [N x dv]: the state before the chunk
+//     S           <- F . S + X2[Q x N]^T (cs . V)            V [Q x dv]: the tokens' values
+// whose operands a thread holds for up to 16 multiply-adds each.  X1 is what the outputs read with,
+// decayed from the chunk's start; X2 what the values are taken in with, decayed to its end; A[i][j] what
+// output i sees of value j.  Decays are always products of the tokens' own decays from j to i (no
+// quotients of running products), so nothing grows and nothing is lost where a decay is zero.  All float32.
+//   state space   X1 = C, X2 = B (shared by a group's heads), rs, cs, A from the heads' scalar decays
+//   delta rule    a decay per row; the removals p solve a unit triangular system within the chunk; with
+//                 its inverse worked into the operands (delta_chunks_kernel) they are Q more rows of the
+//                 first product, and in the second Q more rows against the chunk's -a u
+// A block of 256 threads owns COLS columns of one (head, sequence); the next chunk's operands come by
+// cp.async while this one is multiplied.  What bounds it: the multiply-adds of one block per SM (state
+// space) and the four barriers of a small chunk (delta rule).
+//
+// Measured (B200), us, token by token / by chunks; within 3e-7 of one another:
+//   tokens                               64     255     1024      2048      6000   8 x 750   20 x 100
+//   state space, 64 heads of 128 x 64  32/30  90/46  322/130   628/245  1777/694   977/636    398/320
+//   delta rule, 32 heads of 64 x 64    31/22  93/49  355/155   704/303  2048/862   759/681    258/274
+//   delta rule, 64 heads               33/31 104/71  402/260   794/507 2309/1463 1354/1334    491/526
+// so the state space goes by chunks from 64 tokens of a request, the delta rule while the step has at most
+// 512 walks (requests times heads): beyond, the token walk fills the GPU by itself.
+// (Tried: the forget gate's recurrence this way, chunks of 32: 268 us against 233 token by token.)
+#include "common.cuh"
+
+#define SB_ERR_BAD_SLOT 16
+
+namespace {
+
+constexpr int THREADS = 256;
+
+__device__ __forceinline__ void copy16(float* smem, const float* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+__device__ __forceinline__ void copy8(float* smem, const float* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
+}
+__device__ __forceinline__ void fma4(float (&a)[4], float m, const float4& v) {
+  a[0] = fmaf(m, v.x, a[0]); a[1] = fmaf(m, v.y, a[1]); a[2] = fmaf(m, v.z, a[2]); a[3] = fmaf(m, v.w, a[3]);
+}
+// Four values each summed over the warp in seven shuffles; lane l ends with value (l >> 3 & 3)'s sum.
+__device__ __forceinline__ float warp_sum_four(float a, float b, float c, float d) {
+  const int lane = threadIdx.x & 31;
+  const bool up = lane & 16, odd = lane & 8;
+  const float s0 = up ? a : c, s1 = up ? b : d;
+  float k0 = (up ? c : a) + __shfl_xor_sync(0xffffffffu, s0, 16);
+  float k1 = (up ? d : b) + __shfl_xor_sync(0xffffffffu, s1, 16);
+  float k = (odd ? k1 : k0) + __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+  return k;
+}
+
+struct Walk {
+  const float *x1, *x2;      // row r of a chunk, head h: + (row0 + r) * x_stride + h * x_head
+  long long x_stride, x_head;
+  const float* v;            // token t, head h: + t * v_stride + h * dv
+  long long v_stride;
+  const float* a;            // chunk, head (or group): [R][Q]
+  int a_heads;               // how many of them a chunk has
+  const float* keep;         // chunk, head: [N] (a decay per row); state space: steps [T, H, 2]
+  const float* skip;         // state space: [H]
+  float* state;              // [slots, H, N, dv]
+  float* out;                // [T, H, dv]
+  const int *cu_q, *slots;
+  int num_slots, H, N, dv;
+  int* err;
+};
+
+// The chunks of all sequences have places of their own: chunk c of sequence b is at cu_q[b] / Q + b + c.
+long long chunk_places(long long tokens, int num_seqs, int q) { return tokens / q + num_seqs; }
+
+// Q tokens of a chunk; R rows of the first product (2 Q for the delta rule); NP the state's rows, padded;
+// SCALAR: the state-space form (one decay per token and head; x1 and x2 are rows of tokens, not of chunks).
+template <int Q, int R, int NP, int COLS, bool SCALAR>
+struct Layout {
+  static constexpr int X1_LD = NP + 4, A_LD = Q + 4;  // (the 4: neighbouring rows fall on neighbouring banks)
+  static constexpr int X1 = 0, X2 = X1 + R * X1_LD, V = X2 + R * NP, A = V + Q * COLS, KEEP = A + R * A_LD;
+  static constexpr int STAGE = KEEP + (SCALAR ? 2 * Q : NP);
+  static constexpr int CG = COLS / 4, TILE_THREADS = R / 4 * CG, SPLITS = THREADS / TILE_THREADS;
+  static constexpr int S = 2 * STAGE, PART = S + NP * COLS, VS = PART + SPLITS * R * COLS, RS = VS + R * COLS;
+  static constexpr size_t BYTES = (size_t)(RS + (SCALAR ? 4 * Q + 4 : 0)) * sizeof(float);
+};
+
+template <int Q, int R, int NP, int COLS, bool SCALAR>
+__global__ void __launch_bounds__(THREADS)
+chunk_walk_kernel(const Walk w) {
+  using L = Layout<Q, R, NP, COLS, SCALAR>;
+  constexpr int CG = L::CG, TT = L::TILE_THREADS, SPLITS = L::SPLITS, TR = R / 4;
+  constexpr int SR = NP * COLS / (THREADS * 4);  // rows of the state per thread
+  constexpr int KN = NP / SPLITS, KA = Q / SPLITS < 4 ? 4 : Q / SPLITS;
+  static_assert(KN % 4 == 0 && SR >= 1 && SPLITS >= 1 && (!SCALAR || Q == 64), "");
+  pdl_wait_block();
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) float smem[];
+  const int h = blockIdx.x, b = blockIdx.y, col0 = blockIdx.z * COLS, tid = threadIdx.x;
+  const int first = w.cu_q[b], n = w.cu_q[b + 1] - first;
+  const int slot = w.slots[b];
+  if (slot < 0 || slot >= w.num_slots) {
+    if (tid == 0) atomicOr(w.err, SB_ERR_BAD_SLOT);
+    return;
+  }
+  const int chunks = (n + Q - 1) / Q;
+  const long long place0 = first / Q + b;
+  const int N = w.N, dv = w.dv, a_head = h / (w.H / w.a_heads);
+  const int cols_here = min(COLS, dv - col0);  // (a multiple of four, as N)
+  // rows from N on and columns from the head's last on are never copied: they stay zero
+  if (N < NP || cols_here < COLS) {
+    for (int i = tid; i < 2 * L::STAGE; i += THREADS) smem[i] = 0.f;
+    __syncthreads();
+  }
+
+  auto issue = [&](int which, int chunk) {
+    float* st = smem + which * L::STAGE;
+    const long long place = place0 + chunk;
+    const int at = first + chunk * Q, left = n - chunk * Q - 1;  // (rows behind the last token: that token's again)
+    const long long head = a_head * w.x_head;
+#pragma unroll
+    for (int i0 = 0; i0 < R * NP / 4; i0 += THREADS) {
+      const int i = i0 + tid, r = i / (NP / 4), c = i % (NP / 4) * 4;
+      if (c < N && i < R * NP / 4) {
+        const long long from = (SCALAR ? (long long)(at + min(r, left)) : place * R + r) * w.x_stride + head + c;
+        copy16(st + L::X1 + r * L::X1_LD + c, w.x1 + from);
+        copy16(st + L::X2 + r * NP + c, w.x2 + from);
+      }
+    }
+#pragma unroll
+    for (int i0 = 0; i0 < Q * CG; i0 += THREADS) {
+      const int i = i0 + tid, r = i / CG, c = i % CG * 4;
+      if (c < cols_here && i < Q * CG)
+        copy16(st + L::V + r * COLS + c, w.v + (long long)(at + min(r, left)) * w.v_stride + (long long)h * dv + col0 + c);
+    }
+    const float* a = w.a + (place * w.a_heads + a_head) * (R * Q);
+#pragma unroll
+    for (int i0 = 0; i0 < R * Q / 4; i0 += THREADS) {
+      const int i = i0 + tid, r = i / (Q / 4), c = i % (Q / 4) * 4;
+      if (i < R * Q / 4) copy16(st + L::A + r * L::A_LD + c, a + r * Q + c);
+    }
+    if constexpr (SCALAR) {
+      if (tid < Q) copy8(st + L::KEEP + 2 * tid, w.keep + ((long long)(at + min(tid, left)) * w.H + h) * 2);
+    } else {
+      if (4 * tid < N) copy16(st + L::KEEP + 4 * tid, w.keep + (place * w.H + h) * N + 4 * tid);
+    }
+  };
+
+  if (chunks > 0) issue(0, 0);
+  asm volatile("cp.async.commit_group;\n" ::);
+  float* S = w.state + ((size_t)slot * w.H + h) * N * dv;
+  float* Ss = smem + L::S;
+  float* part = smem + L::PART;
+  float* Vs = smem + L::VS;
+  const int s_col = tid % CG * 4, s_row = tid / CG * SR;
+  float s[SR][4];
+#pragma unroll
+  for (int r = 0; r < SR; ++r) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      s[r][c] = (s_row + r < N && s_col + c < cols_here) ? S[(size_t)(s_row + r) * dv + col0 + s_col + c] : 0.f;
+    *reinterpret_cast<float4*>(Ss + (s_row + r) * COLS + s_col) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
+  }
+  const int split = tid / TT, rg = tid % TT / CG, cg4 = tid % CG * 4;
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    float* st = smem + (chunk & 1) * L::STAGE;
+    const int count = min(Q, n - chunk * Q);
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();  // this chunk's operands and the state stand; the other buffer has been read
+    if (chunk + 1 < chunks) issue((chunk + 1) & 1, chunk + 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    // A value that is not finite must not reach the outputs before it (0 times it is not 0): a chunk with
+    // one masks the values by row.
+    bool odd = false;
+#pragma unroll
+    for (int i0 = 0; i0 < Q * COLS; i0 += THREADS) odd |= !isfinite(st[L::V + i0 + tid]);
+    [[maybe_unused]] float *rs = smem + L::RS, *cs = rs + Q, *own = cs + Q, *dec = own + Q, *block = dec + Q;
+    if constexpr (SCALAR) {
+      // Decays: products within blocks of 16 tokens (scans over 16 lanes), then over the blocks.  own[j]:
+      // those behind j in j's block; block[k]: all of block k.
+      if (tid < Q) {
+        const int l = tid & 15;
+        const float d = tid < count ? st[L::KEEP + 2 * tid] : 1.f;
+        float up = d, down = d;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+          const float a = __shfl_up_sync(0xffffffffu, up, o, 16), z = __shfl_down_sync(0xffffffffu, down, o, 16);
+          if (l >= o) up *= a;
+          if (l + o < 16) down *= z;
+        }
+        const float behind = __shfl_down_sync(0xffffffffu, down, 1, 16);
+        rs[tid] = up;
+        own[tid] = l < 15 ? behind : 1.f;
+        dec[tid] = d;
+        if (l == 15) block[tid >> 4] = up;
+      }
+    }
+    odd = __syncthreads_or(odd);
+    if constexpr (SCALAR) {
+      // A[i][j] = (C_i . B_j) * (decays from j + 1 to i) * dt_j; rs[i] = decays up to i; cs[j] = dt_j * decays after j
+      const int j = tid % Q, bj = j >> 4, bi = tid / Q;  // 16 rows of block bi
+      const float dt = j < count ? st[L::KEEP + 2 * j + 1] : 0.f;
+      float run = bi > bj ? own[j] : 1.f;
+      for (int k = bj + 1; k < bi; ++k) run *= block[k];
+#pragma unroll 8
+      for (int i = 16 * bi; i < 16 * bi + 16; ++i) {
+        if (i > j) run *= dec[i];
+        float* a = st + L::A + i * L::A_LD + j;
+        *a = i >= j ? *a * run * dt : 0.f;
+      }
+      if (bi == 0) {
+        float r = rs[j], c = own[j] * dt;
+        for (int k = 0; k < bj; ++k) r *= block[k];
+        for (int k = bj + 1; k < 4; ++k) c *= block[k];
+        rs[j] = r;
+        cs[j] = c;
+      }
+      __syncthreads();
+    }
+    // ---- rs . (X1 S) + A V, rows rg + TR r and columns cg4 .. of this thread, its slice of the inner sums ----
+    float acc[4][4] = {};
+    {
+      const float* x1 = st + L::X1 + rg * L::X1_LD + split * KN;
+      const float* ss = Ss + split * KN * COLS + cg4;
+#pragma unroll 4
+      for (int k = 0; k < KN; k += 4) {
+        float4 x[4], v[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          x[r] = *reinterpret_cast<const float4*>(x1 + r * TR * L::X1_LD + k);
+          v[r] = *reinterpret_cast<const float4*>(ss + (k + r) * COLS);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          fma4(acc[r], x[r].x, v[0]); fma4(acc[r], x[r].y, v[1]); fma4(acc[r], x[r].z, v[2]); fma4(acc[r], x[r].w, v[3]);
+        }
+      }
+    }
+    if constexpr (SCALAR)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] *= rs[rg + TR * r];
+    if (split * KA < Q) {
+      const float* a = st + L::A + rg * L::A_LD + split * KA;
+      const float* vv = st + L::V + split * KA * COLS + cg4;
+#pragma unroll 4
+      for (int k = 0; k < KA; k += 4) {
+        float4 x[4], v[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          x[r] = *reinterpret_cast<const float4*>(a + r * TR * L::A_LD + k);
+          v[r] = *reinterpret_cast<const float4*>(vv + (k + r) * COLS);
+        }
+        if (odd) {
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float xr[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              if (split * KA + k + kk <= (rg + TR * r) % Q) fma4(acc[r], xr[kk], v[kk]);
+          }
+          continue;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          fma4(acc[r], x[r].x, v[0]); fma4(acc[r], x[r].y, v[1]); fma4(acc[r], x[r].z, v[2]); fma4(acc[r], x[r].w, v[3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      *reinterpret_cast<float4*>(part + (split * R + rg + TR * r) * COLS + cg4) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+    __syncthreads();
+    // ---- the slices' sum: outputs, and the rows that the update takes ----
+    for (int i = tid; i < R * CG; i += THREADS) {
+      const int r = i / CG, c = i % CG * 4;
+      float4 y = *reinterpret_cast<const float4*>(part + r * COLS + c);
+#pragma unroll
+      for (int p = 1; p < SPLITS; ++p) {
+        const float4 z = *reinterpret_cast<const float4*>(part + (p * R + r) * COLS + c);
+        y.x += z.x; y.y += z.y; y.z += z.z; y.w += z.w;
+      }
+      float4 take = y;
+      if (r < Q) {
+        take = *reinterpret_cast<const float4*>(st + L::V + r * COLS + c);
+        if constexpr (SCALAR) {
+          const float d = w.skip[h], f = cs[r];
+          y.x = fmaf(d, take.x, y.x); y.y = fmaf(d, take.y, y.y); y.z = fmaf(d, take.z, y.z); y.w = fmaf(d, take.w, y.w);
+          take.x *= f; take.y *= f; take.z *= f; take.w *= f;
+        }
+        if (r < count && c < cols_here)
+          *reinterpret_cast<float4*>(w.out + ((size_t)(first + chunk * Q + r) * w.H + h) * dv + col0 + c) = y;
+      }
+      *reinterpret_cast<float4*>(Vs + r * COLS + c) = take;
+    }
+    __syncthreads();
+    // ---- S <- F . S + X2^T Vs ----
+#pragma unroll
+    for (int r = 0; r < SR; ++r) {
+      const float keep = SCALAR ? rs[Q - 1] : st[L::KEEP + s_row + r];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) s[r][c] *= keep;
+    }
+    const float* x2 = st + L::X2 + s_row;
+#pragma unroll 8
+    for (int j = 0; j < R; ++j) {
+      const float4 v = *reinterpret_cast<const float4*>(Vs + j * COLS + s_col);
+      float x[SR];
+      if constexpr (SR == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(x2 + j * NP);
+        x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+      } else {
+#pragma unroll
+        for (int r = 0; r < SR; ++r) x[r] = x2[j * NP + r];
+      }
+#pragma unroll
+      for (int r = 0; r < SR; ++r) fma4(s[r], x[r], v);
+    }
+#pragma unroll
+    for (int r = 0; r < SR; ++r)
+      *reinterpret_cast<float4*>(Ss + (s_row + r) * COLS + s_col) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  for (int i = 0; i < b; ++i)
+    if (w.slots[i] == slot) return;  // the slot's first row writes the state
+#pragma unroll
+  for (int r = 0; r < SR; ++r)
+    if (s_row + r < N && s_col < cols_here)
+      *reinterpret_cast<float4*>(S + (size_t)(s_row + r) * dv + col0 + s_col) = make_float4(s[r][0], s[r][1], s[r][2], s[r][3]);
+}
+
+template <int Q, int R, int NP, int COLS, bool SCALAR>
+int launch_walk(const Walk& w, int num_seqs, cudaStream_t stream) {
+  using L = Layout<Q, R, NP, COLS, SCALAR>;
+  static const int configured = (int)cudaFuncSetAttribute(chunk_walk_kernel<Q, R, NP, COLS, SCALAR>,
+                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES);
+  if (configured != 0) return configured;
+  sb_launch_plain(chunk_walk_kernel<Q, R, NP, COLS, SCALAR>, dim3(w.H, num_seqs, (w.dv + COLS - 1) / COLS), THREADS, L::BYTES,
+                  stream, w);
+  SB_LAUNCH_CHECK();
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
+// State space: G[chunk, group][i][j] = C_i . B_j over a chunk's tokens (the heads of a group share it).
+// ---------------------------------------------------------------------------
+constexpr int SSQ = 64, SSN = 128;
+
+__global__ void __launch_bounds__(THREADS)
+state_space_chunks_kernel(const float* __restrict__ xbc, int C, int inner, int G, int N, const int* __restrict__ cu_q,
+                          float* __restrict__ out) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  constexpr int LD = SSN + 4;
+  extern __shared__ __align__(16) float smem[];  // C | B, [SSQ][LD] each
+  const int chunk = blockIdx.x, b = blockIdx.y, g = blockIdx.z, tid = threadIdx.x;
+  const int first = cu_q[b], n = cu_q[b + 1] - first;
+  if (chunk * SSQ >= n) return;
+  const int at = first + chunk * SSQ, left = n - chunk * SSQ - 1, n4 = N >> 2;
+  for (int i = tid; i < SSQ * n4; i += THREADS) {
+    const int r = i / n4, c = (i - r * n4) * 4;
+    const float* row = xbc + (size_t)(at + min(r, left)) * C + inner + c;
+    copy16(smem + r * LD + c, row + (size_t)(G + g) * N);
+    copy16(smem + (SSQ + r) * LD + c, row + (size_t)g * N);
+  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::);
+  __syncthreads();
+  const int tr = tid >> 4, tc = tid & 15;  // rows tr + 16 r, columns tc + 16 c
+  float acc[4][4] = {};
+#pragma unroll 2
+  for (int k = 0; k < N; k += 4) {
+    float4 x[4], y[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      x[r] = *reinterpret_cast<const float4*>(smem + (tr + 16 * r) * LD + k);
+      y[r] = *reinterpret_cast<const float4*>(smem + (SSQ + tc + 16 * r) * LD + k);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        acc[r][c] = fmaf(x[r].x, y[c].x, acc[r][c]);
+        acc[r][c] = fmaf(x[r].y, y[c].y, acc[r][c]);
+        acc[r][c] = fmaf(x[r].z, y[c].z, acc[r][c]);
+        acc[r][c] = fmaf(x[r].w, y[c].w, acc[r][c]);
+      }
+  }
+  float* to = out + ((long long)(first / SSQ + b + chunk) * G + g) * (SSQ * SSQ);
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) to[(tr + 16 * r) * SSQ + tc + 16 * c] = acc[r][c];
+}
+
+// ---------------------------------------------------------------------------
+// Delta rule: a block per chunk and head, from the projections (general_delta_inputs_kernel in state_scans.cu
+// names them): w, u, a u, k, r per token and channel, and vals [T, H, d].  With D(j, i) the decays of the
+// tokens j + 1 .. i:  p_i = u_i . S_{i-1} gives (I + T) p = U S + K V with
+//   T[i][j] = u_i D(j, i-1) (a u)_j,  K[i][j] = u_i D(j, i-1) k_j  (j < i),  U_i = u_i D(0, i-1)
+// and o_i = r_i D(0, i) S + sum over j <= i of (r_i D(j, i) k_j) v_j - (r_i D(j, i) (a u)_j) p_j.  With
+// U' = (I + T)^-1 U, K' = (I + T)^-1 K and Ra[i][j] = r_i D(j, i) (a u)_j:
+//   x1 = [r_i D(0, i) - Ra U' ; U'],  a = [r_i D(j, i) k_j - Ra K' ; K'],  x2 = [k_j D(j, Q) ; -(a u)_j D(j, Q)]
+// ---------------------------------------------------------------------------
+constexpr int GDQ = 16, GDN = 64;
+
+__global__ void __launch_bounds__(THREADS)
+delta_chunks_kernel(const bf16* __restrict__ pre, int pre_width, const bf16* __restrict__ low, int low_width,
+                    const float* __restrict__ decay_bias, const float* __restrict__ removal_bias, int H, int d,
+                    const int* __restrict__ cu_q, float* __restrict__ vals, float* __restrict__ x1, float* __restrict__ x2,
+                    float* __restrict__ keep, float* __restrict__ a) {
+  pdl_wait_block();
+  pdl_launch_dependents();
+  __shared__ float in[5][GDQ][GDN];                                   // w, u, a u, k, r
+  __shared__ float t_s[GDQ][GDQ], k_s[GDQ][GDQ], rk_s[GDQ][GDQ], ra_s[GDQ][GDQ];
+  __shared__ float u_s[GDQ][GDN + GDQ], x_s[GDQ][GDN + GDQ];          // U' | K';  r D(0, i) | r D k
+  const int chunk = blockIdx.x, b = blockIdx.y, h = blockIdx.z, tid = threadIdx.x;
+  const int first = cu_q[b], n = cu_q[b + 1] - first;
+  if (chunk * GDQ >= n) return;
+  const int at = first + chunk * GDQ, count = min(GDQ, n - chunk * GDQ), inner = H * d;
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int i = warp + 8 * half, t = at + min(i, count - 1);
+    const bf16* row = pre + (size_t)t * pre_width + (size_t)h * d;
+    const bf16* lrow = low + (size_t)t * low_width + (size_t)h * d;
+    const bool live = i < count;
+    float k[2], z[2] = {0.f, 0.f}, l[2] = {0.f, 0.f}, r[2] = {0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = lane + 32 * q;
+      k[q] = live && c < d ? to_f32<bf16>(row[inner + c]) : 0.f;
+      if (live && c < d) {
+        r[q] = to_f32<bf16>(row[c]);
+        z[q] = to_f32<bf16>(row[4 * inner + c]) + removal_bias[h * d + c];
+        l[q] = to_f32<bf16>(lrow[c]) + decay_bias[h * d + c];
+        vals[((size_t)t * H + h) * d + c] = to_f32<bf16>(row[2 * inner + c]);
+      }
+    }
+    const float inv = 1.0f / sqrtf(warp_sum(fmaf(k[0], k[0], k[1] * k[1])) + 1e-6f);
+    const float rate = 0.6065306597126334f;  // e^(-1/2)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = lane + 32 * q;
+      const bool on = live && c < d;
+      const float u = k[q] * inv;
+      in[0][i][c] = on ? expf(-rate / (1.0f + expf(-l[q]))) : 1.f;
+      in[1][i][c] = u;
+      in[2][i][c] = on ? u / (1.0f + expf(-z[q])) : 0.f;
+      in[3][i][c] = k[q];
+      in[4][i][c] = r[q];
+    }
+  }
+  t_s[tid / GDQ][tid % GDQ] = k_s[tid / GDQ][tid % GDQ] = rk_s[tid / GDQ][tid % GDQ] = ra_s[tid / GDQ][tid % GDQ] = 0.f;
+  __syncthreads();
+  const long long place = first / GDQ + b + chunk;
+  float* const sums[4] = {&t_s[0][0], &k_s[0][0], &rk_s[0][0], &ra_s[0][0]};
+  float* const mine = sums[lane >> 3];
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int j = half ? GDQ - 1 - warp : warp;  // (a long and a short column per warp)
+    float k0 = in[3][j][lane], k1 = in[3][j][lane + 32], a0 = in[2][j][lane], a1 = in[2][j][lane + 32];
+#pragma unroll 2
+    for (int i = j; i < GDQ; ++i) {
+      float t = 0.f, kk = 0.f;
+      if (i > j) {
+        const float u0 = in[1][i][lane], u1 = in[1][i][lane + 32], w0 = in[0][i][lane], w1 = in[0][i][lane + 32];
+        t = fmaf(u0, a0, u1 * a1);
+        kk = fmaf(u0, k0, u1 * k1);
+        k0 *= w0; k1 *= w1; a0 *= w0; a1 *= w1;
+      }
+      const float r0 = in[4][i][lane], r1 = in[4][i][lane + 32];
+      const float sum = warp_sum_four(t, kk, fmaf(r0, k0, r1 * k1), fmaf(r0, a0, r1 * a1));
+      if ((lane & 7) == 0) mine[i * GDQ + j] = sum;
+    }
+  }
+  __syncthreads();
+  // a thread per column of U | K: forward substitution; beside it the decays of r, k and a u
+  const size_t x_row = (size_t)H * d, x_at = (size_t)place * 2 * GDQ * x_row + (size_t)h * d;
+  if (tid < GDN + GDQ) {
+    const int c = tid;
+    float col[GDQ], run = 1.f;
+#pragma unroll
+    for (int i = 0; i < GDQ; ++i) {
+      if (c < GDN) {
+        col[i] = in[1][i][c] * run;
+        run *= in[0][i][c];
+        x_s[i][c] = in[4][i][c] * run;
+      } else {
+        col[i] = k_s[i][c - GDN];
+        x_s[i][c] = rk_s[i][c - GDN];
+      }
+    }
+#pragma unroll
+    for (int i = 1; i < GDQ; ++i)
+#pragma unroll
+      for (int j = 0; j < i; ++j) col[i] = fmaf(-t_s[i][j], col[j], col[i]);
+#pragma unroll
+    for (int i = 0; i < GDQ; ++i) u_s[i][c] = col[i];
+    if (c < d) keep[(place * H + h) * d + c] = run;
+  } else if (tid >= 128 && tid - 128 < d) {
+    const int c = tid - 128;
+    float run = 1.f;
+#pragma unroll 4
+    for (int i = GDQ - 1; i >= 0; --i) {
+      x2[x_at + i * x_row + c] = in[3][i][c] * run;
+      x2[x_at + (GDQ + i) * x_row + c] = -in[2][i][c] * run;
+      run *= in[0][i][c];
+    }
+  }
+  __syncthreads();
+  float* a_to = a + (place * H + h) * (2 * GDQ * GDQ);
+#pragma unroll
+  for (int m = 0; m < GDQ * (GDN + GDQ) / THREADS; ++m) {
+    const int idx = tid + m * THREADS, i = idx / (GDN + GDQ), c = idx % (GDN + GDQ);
+    float v = x_s[i][c];
+    for (int j = 0; j <= i; ++j) v = fmaf(-ra_s[i][j], u_s[j][c], v);
+    if (c >= GDN) {
+      a_to[i * GDQ + c - GDN] = v;
+      a_to[(GDQ + i) * GDQ + c - GDN] = u_s[i][c];
+    } else if (c < d) {
+      x1[x_at + i * x_row + c] = v;
+      x1[x_at + (GDQ + i) * x_row + c] = u_s[i][c];
+    }
+  }
+}
+
+bool aligned16(const void* a, const void* b, const void* c) { return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) == 0; }
+
+}  // namespace
+
+// Whether a walk by chunks takes the shape, and the floats of its workspace (0: it does not).
+// kind 0 state space (heads: groups, d: state rows, dv: a head's values, other: floats per row of xbc), 1 delta rule.
+extern "C" long long sb_chunk_walk_floats(int kind, long long tokens, int num_seqs, int heads, int d, int dv, int other) {
+  if (d <= 0 || d % 4 || dv % 4) return 0;
+  if (kind == 0) return d <= SSN && other % 4 == 0 ? chunk_places(tokens, num_seqs, SSQ) * heads * SSQ * SSQ : 0;
+  if (d > GDN) return 0;
+  const long long per_chunk = 4LL * GDQ * d + d + 2LL * GDQ * GDQ;
+  return (chunk_places(tokens, num_seqs, GDQ) * per_chunk + tokens * d) * heads;
+}
+
+extern "C" int sb_chunk_state_space(const float* xbc, int C, const float* steps, const float* skip, float* state,
+                                    const int* cu_q, const int* slots, int num_seqs, int num_slots, int H, int G, int N, int dv,
+                                    int max_q_len, float* scratch, float* out, int* err, cudaStream_t stream) {
+  if (!aligned16(xbc, state, out) || !aligned16(scratch, out, out)) return -13;
+  const int inner = H * dv;
+  constexpr size_t smem = (size_t)2 * SSQ * (SSN + 4) * sizeof(float);
+  static const int configured =
+      (int)cudaFuncSetAttribute(state_space_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (configured != 0) return configured;
+  sb_launch(state_space_chunks_kernel, dim3((max_q_len + SSQ - 1) / SSQ, num_seqs, G), THREADS, smem, stream, xbc, C, inner, G, N,
+            cu_q, scratch);
+  SB_LAUNCH_CHECK();
+  const Walk w{xbc + inner + (size_t)G * N, xbc + inner, C, N, xbc, C, scratch, G, steps, skip, state, out, cu_q, slots,
+               num_slots, H, N, dv, err};
+  return launch_walk<SSQ, SSQ, SSN, 32, true>(w, num_seqs, stream);
+}
+
+// pre, low: bfloat16, as sb_general_delta_scan takes them.
+extern "C" int sb_chunk_delta(const void* pre, int pre_width, const void* low, int low_width, const float* decay_bias,
+                              const float* removal_bias, float* state, const int* cu_q, const int* slots, int num_tokens,
+                              int num_seqs, int num_slots, int H, int d, int max_q_len, float* scratch, float* out, int* err,
+                              cudaStream_t stream) {
+  if (num_seqs == 0 || num_tokens == 0) return 0;
+  if (d <= 0 || d % 4 || d > GDN || !aligned16(state, out, scratch)) return -13;
+  const long long places = chunk_places(num_tokens, num_seqs, GDQ), rows = places * 2 * GDQ * H * d;
+  float *x1 = scratch, *x2 = x1 + rows, *keep = x2 + rows, *a = keep + places * H * d, *vals = a + places * H * 2 * GDQ * GDQ;
+  sb_launch(delta_chunks_kernel, dim3((max_q_len + GDQ - 1) / GDQ, num_seqs, H), THREADS, 0, stream, (const bf16*)pre, pre_width,
+            (const bf16*)low, low_width, decay_bias, removal_bias, H, d, cu_q, vals, x1, x2, keep, a);
+  SB_LAUNCH_CHECK();
+  const Walk w{x1, x2, (long long)H * d, d, vals, (long long)H * d, a, H, keep, nullptr, state, out, cu_q, slots, num_slots, H, d, d, err};
+  return launch_walk<GDQ, 2 * GDQ, GDN, 16, false>(w, num_seqs, stream);
+}

@@ -751,12 +751,17 @@ state_space_patch_kernel(const float* __restrict__ xbc, int C, const float* __re
   }
 }
 
-// scratch: float32 [T, H, 2].
+extern "C" int sb_chunk_state_space(const float* xbc, int C, const float* steps, const float* skip, float* state,
+                                    const int* cu_q, const int* slots, int num_seqs, int num_slots, int H, int G, int N, int dv,
+                                    int max_q_len, float* scratch, float* out, int* err, cudaStream_t stream);
+
+// scratch: float32 [T, H, 2].  chunk_scratch: null, or what the walk by chunks needs (chunk_walks.cu).
 extern "C" int sb_state_space_scan(const float* xbc, int C, const void* pre, int pre_width, int dtype,
                                    int step_offset, const float* step_bias, const float* neg_rate,
                                    const float* skip, float* state, const int* cu_q, const int* slots,
                                    int num_tokens, int num_seqs, int num_slots, int H, int G, int N, int dv,
-                                   int max_q_len, float* scratch, float* out, int* err, cudaStream_t stream) {
+                                   int max_q_len, float* scratch, float* chunk_scratch, float* out, int* err,
+                                   cudaStream_t stream) {
   if (num_seqs == 0 || num_tokens == 0) return 0;
   if (N <= 0 || N > 1024 || dv <= 0 || H <= 0 || G <= 0 || H % G) return -13;
   const long long total = (long long)num_tokens * H;
@@ -768,6 +773,9 @@ extern "C" int sb_state_space_scan(const float* xbc, int C, const void* pre, int
     sb_launch(state_space_steps_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)pre, pre_width, step_offset,
               step_bias, neg_rate, H, total, scratch);
   SB_LAUNCH_CHECK();
+  if (chunk_scratch != nullptr)
+    return sb_chunk_state_space(xbc, C, scratch, skip, state, cu_q, slots, num_seqs, num_slots, H, G, N, dv, max_q_len,
+                                chunk_scratch, out, err, stream);
   const bool long_walk = max_q_len >= 64;
   if (long_walk && N >= 16 && N <= 128) {
     int rg = 4;

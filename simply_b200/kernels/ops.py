@@ -190,6 +190,10 @@ class CudaOps:
     # tile: 0 128, 1 256, -1 the launch chooses (tests).  Where the lines lie: sb_moe_grouped_tc.
     self.experts_pair_rows = 64
     self.experts_wide = -1
+    # From how many tokens of a request a step's walks through recurrent states go by chunks of tokens: the
+    # state-space recurrence, the generalized delta rule; 0 never (tests).
+    self.chunk_walk_tokens = [64, 64]
+    self.chunk_walk_most = 512  # ... and up to how many walks of the delta rule at once (csrc/chunk_walks.cu)
     self._wide_tables: dict[tuple, torch.Tensor] = {}
     self.prefill_single_key_group = False  # True: 64-row tiles with 4 warps instead of 4 x 2 (experiments, tests)
     # 0: the weight-streaming product picks its warps per block; 4, 8 or 16 forces them (experiments).
@@ -311,7 +315,9 @@ class CudaOps:
                                   c_int, c_int, c_int, c_int, c_int, c_void, c_void, c_void, c_void],
         "sb_state_space_scan": [c_void, c_int, c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_void,
                                 c_void, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void, c_void,
-                                c_void, c_void],
+                                c_void, c_void, c_void],
+        "sb_chunk_delta": [c_void, c_int, c_void, c_int, c_void, c_void, c_void, c_void, c_void, c_int, c_int, c_int,
+                           c_int, c_int, c_int, c_void, c_void, c_void, c_void],
         "sb_forget_scan": [c_void, c_int, c_int, c_void, c_void, c_void, c_void, c_void, c_int, c_int, c_int, c_int,
                            c_int, c_int, c_int, c_void, c_void, c_void, c_void],
         "sb_moe_route": [c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_int, c_int, c_float, c_int, c_int,
@@ -345,6 +351,8 @@ class CudaOps:
     self.lib.sb_gemm_library_bf16_heads.argtypes = [c_void, c_int, c_int, c_void, c_void, c_int, c_int, c_int, c_int, c_int,
                                                     c_int, ctypes.c_float, c_void, c_ll, c_void]
     self.lib.sb_gemm_library_bf16_heads.restype = c_int
+    self.lib.sb_chunk_walk_floats.argtypes = [c_int, c_ll, c_int, c_int, c_int, c_int, c_int]
+    self.lib.sb_chunk_walk_floats.restype = c_ll
     self.lib.sb_graph_burst.argtypes = [c_void, c_void, c_void, c_ll, c_int, c_void, c_void, c_ll, c_void]
     self.lib.sb_graph_burst.restype = c_int
     self.lib.sb_stream_wait.argtypes = [c_void]
@@ -1423,6 +1431,18 @@ class CudaOps:
     return out
 
   # ---- recurrent mixers with a matrix per head ------------------------------------------------------
+  def _chunk_scratch(self, kind: int, ctx: Any, tokens: int, heads: int, dim: int, value_dim: int,
+                     other: int = 0) -> torch.Tensor | None:
+    """Workspace of a walk by chunks of tokens (csrc/chunk_walks.cu), or None where a step's walks go token
+    by token: short portions, shapes it does not take, and the 32-bit engine, whose sums do not depend on how
+    a sequence is cut into steps."""
+    if self.dtype != torch.bfloat16 or not 0 < self.chunk_walk_tokens[kind] <= ctx.max_q_len:
+      return None
+    if kind == 1 and ctx.num_seqs * heads > self.chunk_walk_most:
+      return None
+    floats = self.lib.sb_chunk_walk_floats(kind, tokens, ctx.num_seqs, heads, dim, value_dim, other)
+    return self._new(floats, dtype=torch.float32) if floats else None
+
   def general_delta_scan(self, pre: torch.Tensor, low: torch.Tensor, decay_bias: torch.Tensor,
                          removal_bias: torch.Tensor, state: torch.Tensor, ctx: Any, *, num_heads: int,
                          head_dim: int) -> torch.Tensor:
@@ -1430,6 +1450,13 @@ class CudaOps:
     walks every sequence's tokens through its state [slots, heads, head_dim, head_dim] (csrc/state_scans.cu)."""
     t = pre.shape[0]
     out = self._new(t, num_heads, head_dim, dtype=torch.float32)
+    chunks = self._chunk_scratch(1, ctx, t, num_heads, head_dim, head_dim)
+    if chunks is not None:
+      self._call("sb_chunk_delta", _ptr(pre), pre.shape[1], _ptr(low), low.shape[1], _ptr(decay_bias), _ptr(removal_bias),
+                 _ptr(state), _ptr(ctx.cu_q), _ptr(ctx.slots), t, ctx.num_seqs, state.shape[0], num_heads, head_dim,
+                 ctx.max_q_len, _ptr(chunks), _ptr(out), _ptr(self.err))
+      self.launches += 1
+      return out
     scratch = self._new(t, num_heads * (6 * head_dim + 2), dtype=torch.float32)
     self._call("sb_general_delta_scan", _ptr(pre), pre.shape[1], _ptr(low), low.shape[1], _code(pre), _ptr(decay_bias),
                _ptr(removal_bias), _ptr(state), _ptr(ctx.cu_q), _ptr(ctx.slots), t, ctx.num_seqs, state.shape[0],
@@ -1445,11 +1472,12 @@ class CudaOps:
     t = xbc.shape[0]
     out = self._new(t, num_heads, value_dim, dtype=torch.float32)
     scratch = self._new(t, num_heads * 2, dtype=torch.float32)
+    chunks = self._chunk_scratch(0, ctx, t, num_groups, state_dim, value_dim, xbc.shape[1])
     self._call("sb_state_space_scan", _ptr(xbc), xbc.shape[1], _ptr(pre), pre.shape[1], _code(pre), step_offset,
                _ptr(step_bias), _ptr(neg_rate), _ptr(skip), _ptr(state), _ptr(ctx.cu_q), _ptr(ctx.slots), t,
                ctx.num_seqs, state.shape[0], num_heads, num_groups, state_dim, value_dim, ctx.max_q_len,
-               _ptr(scratch), _ptr(out), _ptr(self.err))
-    self.launches += 1
+               _ptr(scratch), _ptr(chunks), _ptr(out), _ptr(self.err))
+    self.launches += 1 + (chunks is not None)
     return out
 
   # ---- forget-gate recurrence ---------------------------------------------------

@@ -744,3 +744,52 @@ def test_grouped_experts_on_tcgen05(table, gated, act, width, hidden, tokens):
   finally:
     ops.experts_pair_rows, ops.experts_wide = before
   ops.check_errors()
+
+
+def _walk_step(lengths):
+  cu = torch.tensor([0, *np.cumsum(lengths)], dtype=torch.int32, device="cuda")
+  return types.SimpleNamespace(max_q_len=max(lengths), num_seqs=len(lengths), cu_q=cu,
+                               slots=torch.arange(len(lengths), dtype=torch.int32, device="cuda").flip(0).contiguous())
+
+
+@pytest.mark.parametrize("odd", [None, math.inf, math.nan])
+@pytest.mark.parametrize("kind,heads,groups,rows,cols", [
+    ("space", 4, 1, 128, 64), ("space", 6, 2, 20, 40), ("space", 2, 1, 64, 4), ("delta", 3, 1, 64, 64), ("delta", 2, 1, 20, 20)])
+@pytest.mark.parametrize("lengths", [[64], [1, 65, 0, 16], [200, 127], [513]])
+def test_walks_by_chunks_match_walks_by_tokens(table, lengths, kind, heads, groups, rows, cols, odd):
+  """A walk by chunks of tokens against the walk token by token: chunks that end anywhere, states smaller
+  than a block's, decays that are zero, and a value that is not finite: what stands before it stays."""
+  ops, ctx, tokens = table[torch.bfloat16], _walk_step(lengths), sum(lengths)
+  gen = torch.Generator(device="cuda").manual_seed(tokens + rows)
+  make = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+  where = int(ctx.cu_q[-2]) + lengths[-1] // 2  # (of the last request)
+  start = make(len(lengths), heads, rows, cols)
+  if kind == "space":
+    xbc, pre = make(tokens, heads * cols + 2 * groups * rows), make(tokens, heads).to(torch.bfloat16)
+    pre[5 % tokens] = 200.0  # a decay of zero
+    if odd is not None:
+      xbc[where, :heads * cols] = odd
+    bias, rate, skip = make(heads) - 2.0, -torch.exp(make(heads)), make(heads)
+    run = lambda state: ops.state_space_scan(xbc, pre, 0, bias, rate, skip, state, ctx, num_heads=heads, value_dim=cols,
+                                             state_dim=rows, num_groups=groups)
+  else:
+    pre, low = make(tokens, 5 * heads * rows).to(torch.bfloat16), (2 * make(tokens, heads * rows)).to(torch.bfloat16)
+    if odd is not None:
+      pre[where, 2 * heads * rows:3 * heads * rows] = odd
+    run = lambda state: ops.general_delta_scan(pre, low, make_bias, make_bias, state, ctx, num_heads=heads, head_dim=rows)
+    make_bias = make(heads * rows)
+  before, got = ops.chunk_walk_tokens, []
+  try:
+    for least in (0, 1):
+      ops.chunk_walk_tokens = [least, least]
+      state = start.clone()
+      got.append((run(state), state))
+  finally:
+    ops.chunk_walk_tokens = before
+  ops.check_errors()
+  for want, have in zip(*got):
+    assert torch.equal(torch.isfinite(want), torch.isfinite(have))
+    keep = torch.isfinite(want)
+    # the same float32 sums of at most 192 products in another order: 2^-24 each, and what a delta rule's
+    # triangular system of 16 adds
+    assert ((want - have)[keep].norm() <= 5e-6 * want[keep].norm()).item()
