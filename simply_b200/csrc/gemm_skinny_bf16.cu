@@ -297,6 +297,9 @@ static int skinny_dispatch(const void* x, const void* w, void* out, int M, int N
   // (4, 8 or 16) is for experiments.
   const int blocks = (n_out + 15) / 16;
   int warps = blocks <= 148 ? 16 : blocks <= 296 ? 8 : 4;
+  // Two token tiles of gate and up rows: with 4 warps a block's loads wait on its own products (9 rows,
+  // us: 18,432 x 2,304 23.8 with 4 warps, 17.3 with 8; 28,672 x 4,096 58.5 and 49.8; 16,384 x 2,048 20.9 and 14.8).
+  if (epilogue == 2 && M > 8 && warps == 4) warps = 8;
   if (K < warps * 32 * 4) warps = K >= 8 * 32 * 4 ? 8 : 4;  // every warp should have a full batch of loads
   if (warps_override == 4 || warps_override == 8 || warps_override == 16) warps = warps_override;
   if (M <= 8) {

@@ -813,8 +813,9 @@ class CudaOps:
       return out
     x = self.cast(x, torch.bfloat16)
     chunk = 32
-    if chunk < r <= self.mid_rows["head"] and self.mid_rows_kernel and k % 8 == 0 and x.is_contiguous():
-      # 33 to 128 rows: one pass over the table instead of several
+    if self.skinny_max_rows < r <= self.mid_rows["head"] and self.mid_rows_kernel and k % 8 == 0 and x.is_contiguous():
+      # The serving batch's kernel from 17 rows (256,000 x 2,304, us: 17 rows 332 through the kernel for a handful of
+      # tokens, 220 here; 32 rows 360 and 237; at 16 rows the two meet, 228 and 218).
       if self._mid_product(x, table, out, 1, cap=cap, split=1):
         return out
     if r > chunk and k % 8 == 0:
