@@ -793,3 +793,42 @@ def test_walks_by_chunks_match_walks_by_tokens(table, lengths, kind, heads, grou
     # the same float32 sums of at most 192 products in another order: 2^-24 each, and what a delta rule's
     # triangular system of 16 adds
     assert ((want - have)[keep].norm() <= 5e-6 * want[keep].norm()).item()
+
+
+@pytest.mark.parametrize("heads,groups,rows,cols", [(4, 1, 128, 64), (3, 1, 64, 16), (2, 2, 8, 128), (2, 1, 32, 256), (2, 1, 12, 64)])
+@pytest.mark.parametrize("requests", [1, 5])
+def test_state_space_step_of_single_tokens(table, heads, groups, rows, cols, requests):
+  """One token per request: the bfloat16 engine's kernel for such steps against the walk that the 32-bit engine
+  keeps, for every number of rows per thread, with a slot that two rows share (the first row's work counts)."""
+  ctx = _walk_step([1] * requests)
+  if requests > 1:
+    ctx.slots[-1] = ctx.slots[-2]
+  gen = torch.Generator(device="cuda").manual_seed(rows * cols)
+  make = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+  xbc, pre = make(requests, heads * cols + 2 * groups * rows), make(requests, heads).to(torch.bfloat16)
+  if requests > 1:
+    xbc[-1], pre[-1] = xbc[-2], pre[-2]
+  start, bias, rate, skip = make(requests, heads, rows, cols), make(heads), -torch.exp(make(heads)), make(heads)
+  got = []
+  for dtype, p in ((torch.float32, pre.float()), (torch.bfloat16, pre)):
+    state = start.clone()
+    out = table[dtype].state_space_scan(xbc, p, 0, bias, rate, skip, state, ctx, num_heads=heads, value_dim=cols,
+                                        state_dim=rows, num_groups=groups)
+    table[dtype].check_errors()
+    got.append((out, state))
+  for want, have in zip(*got):  # sums of at most 128 float32 products in another order: 2^-24 each, and the sum's size
+    assert ((want - have).norm() <= 2e-6 * want.norm()).item()
+
+
+@pytest.mark.parametrize("tokens", [591, 592, 595])
+@pytest.mark.parametrize("width,experts", [(64, 5), (72, 34), (33, 3)])
+def test_route_with_tokens_together(table, tokens, width, experts):
+  """Four tokens per block give what one gives, bit for bit, at the line between them and in a ragged last block."""
+  ops = table[torch.bfloat16]
+  gen = torch.Generator(device="cuda").manual_seed(tokens + width)
+  make = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+  x, router, gate = make(tokens, width).to(torch.bfloat16), make(experts, width), make(width)
+  whole = ops.route_tokens(x, router, None, gate, top=2, scale=1.5)
+  parts = [ops.route_tokens(x[at:at + 100].contiguous(), router, None, gate, top=2, scale=1.5) for at in range(0, tokens, 100)]
+  for i, want in enumerate(whole):
+    assert torch.equal(want, torch.cat([p[i] for p in parts]))
