@@ -832,3 +832,42 @@ def test_route_with_tokens_together(table, tokens, width, experts):
   parts = [ops.route_tokens(x[at:at + 100].contiguous(), router, None, gate, top=2, scale=1.5) for at in range(0, tokens, 100)]
   for i, want in enumerate(whole):
     assert torch.equal(want, torch.cat([p[i] for p in parts]))
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
+@pytest.mark.parametrize("taps,channels,offset,residual,activation,wide", [(3, 64, 0, True, 0, False), (4, 1100, 8, False, 1, True),
+                                                                          (2, 36, 4, False, 0, False)])
+def test_short_convolution_of_many_tokens(table, dtype, taps, channels, offset, residual, activation, wide):
+  """Eight tokens per thread give what one gives, bit for bit: requests that begin anywhere among the eight, requests
+  of no tokens and of fewer than the window, a ragged last group."""
+  ops, lengths = table[dtype], [1, 3, 0, 130, 2, 117, 10]
+  gen = torch.Generator(device="cuda").manual_seed(channels)
+  make = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+  tokens = sum(lengths)
+  x, weight, bias = make(tokens, channels + 2 * offset).to(dtype), make(channels, taps), make(channels)
+  start = make(len(lengths), taps - 1, channels)
+  whole = _walk_step(lengths)
+  whole.token_seq = torch.repeat_interleave(torch.arange(len(lengths), device="cuda"), torch.tensor(lengths, device="cuda")).int()
+  run = lambda x, state, ctx: ops.short_conv(x, weight, bias, state, ctx, activation=activation, residual=residual,
+                                             offset=offset, channels=channels, out_dtype=torch.float32 if wide else None)
+  state = start.clone()
+  got = run(x, state, whole)
+  one_by_one, want = start.clone(), []
+  for i, n in enumerate(lengths):
+    if n == 0:
+      continue
+    at = int(whole.cu_q[i])
+    ctx = _walk_step([n])
+    ctx.slots, ctx.token_seq = whole.slots[i:i + 1].contiguous(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    want.append(run(x[at:at + n].contiguous(), one_by_one, ctx))
+  ops.check_errors()
+  assert torch.equal(got, torch.cat(want)) and torch.equal(state, one_by_one)
+
+
+@pytest.mark.parametrize("rows", [16, 17, 24, 32, 33])
+def test_output_layer_of_a_serving_batch(table, rows):
+  """The lines between the three products that serve the output layer (see test_lm_head for the bound)."""
+  ops, ref = table[torch.bfloat16], ReferenceOps(torch.bfloat16)
+  x, t = (torch.randn(rows, 264) * 2).to(torch.bfloat16), torch.randn(1003, 264).to(torch.bfloat16)
+  torch.testing.assert_close(ops.lm_head(x.cuda(), t.cuda(), 30.0).cpu(), ref.lm_head(x, t, 30.0), atol=2e-4 * 264 ** 0.5, rtol=1e-4)
+  ops.check_errors()
