@@ -1,15 +1,17 @@
 // True 32-bit matrix product on CUDA cores: out[M, N] = x[M, K] . w[N, K]^T.
 //
 // No tensor-core mode, no reduced-precision staging: every product and sum is a
-// float32 FMA.  Every output is one chain of FMAs over k = 0, 1, ..., K - 1, whatever tile
-// computes it, so a token's result does not depend on what else is in the batch.
+// float32 FMA.  Every output is the sum ((c0 + c1) + c2) + c3 of four chains of FMAs, one over each quarter of k
+// (whole tiles of 32 long), whatever kernel computes it and whether the quarters are walked one after the other or
+// side by side, so a token's result does not depend on what else is in the batch.
 // Optional epilogue: soft cap (simply/model_lib.py:107-109) for the output layer.
 //
 // Bound by the FMA pipes for many rows, by the weights' bytes for a few.  Four tile shapes share the
 // chains' order: 128 x 128 outputs (16 x 8 per thread, packed FMAs) for products of many tiles and long rows,
 // 64 x 64 (8 x 4 per thread) where those fill the GPU, 32 x 32 (4 x 4 per thread) where they do not, and
 // 8 x 16 or 16 x 8 (one output per thread) fed by a deep ring of asynchronous copies for up to 16 rows, where
-// the weights only stream by.  sb_gemm_f32_tile has the lines between them.
+// the weights only stream by.  sb_gemm_f32_tile has the lines between them; sb_gemm_f32_groups says whether a
+// tile's quarters of k are four groups of a block's threads.
 #include "common.cuh"
 
 // Two FMAs in one instruction, each rounded as fmaf rounds.
@@ -44,42 +46,58 @@ __device__ __forceinline__ float4 row_quad(const float* __restrict__ p, bool in,
 // row's 16-byte quads; the rows of the four k of quad q are kept at places row ^ turn(q), so that the
 // 32 values a warp stores at a time lie on 32 banks.
 //
+// GROUPS 4: four groups of threads take a quarter of k each, with tiles of their own in shared memory, and their
+// chains meet there at the end; 1: one group walks the quarters in turn and keeps the sum so far there.
+//
 // What bounds it: a warp's reads of shared memory deliver 128 bytes a cycle and SM, so TM + TN cycles per
 // k beside TM TN / 4 cycles of FMAs: 16 x 8 outputs per thread keep the FMA pipes the longer of the two,
-// 8 x 8 are even, and 8 x 4 are half as long again as their FMAs (taken where larger tiles would leave SMs idle).
+// 8 x 8 are even, and 8 x 4 are half as long again as their FMAs.  64 x 64 of 8 x 4 all the same, whose blocks of
+// 128 threads stand four to an SM: with 8 x 8 per thread 256 x 16,384 x 2,048 took 425 us (G = 4: 467) in place of 358.
 // ---------------------------------------------------------------------------
-template <int BM, int BN, int BK, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+// A quarter of k, in whole tiles of 32.
+__host__ __device__ __forceinline__ int f32_quarter(int K) { return (K + 127) / 128 * 32; }
+
+template <int BM, int BN, int BK, int TM, int TN, int GROUPS>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN) * GROUPS)
 gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out, int M, int N,
                      int K, float cap, int vec) {
-  constexpr int THREADS = (BM / TM) * (BN / TN), QUADS = BK / 4;
+  constexpr int THREADS = (BM / TM) * (BN / TN), QUADS = BK / 4;  // (threads of a group)
+  constexpr int TILE_FLOATS = 2 * BK * (BM + BN);  // a group's two tiles of x and of w
+  static_assert(TILE_FLOATS >= BM * BN || GROUPS == 1, "a group's results take the place of its tiles");
   constexpr int XQ = BM * QUADS / THREADS, WQ = BN * QUADS / THREADS;  // quads a thread fetches per tile
   static_assert(BM * QUADS % THREADS == 0 && BN * QUADS % THREADS == 0, "whole quads per thread");
   static_assert(TM % 4 == 0 && TN % 4 == 0 && QUADS <= 8 && BM % 32 == 0 && BN % 32 == 0, "vectors of 4, places within a row");
   pdl_wait_block();
   pdl_launch_dependents();
-  __shared__ __align__(16) float xs[2][BK][BM];
-  __shared__ __align__(16) float ws[2][BK][BN];
+  extern __shared__ __align__(16) float tile_smem[];
+  const int group = GROUPS == 1 ? 0 : threadIdx.x / THREADS, tid = GROUPS == 1 ? threadIdx.x : threadIdx.x % THREADS;
+  float (*xs)[BK][BM] = reinterpret_cast<float (*)[BK][BM]>(tile_smem + group * TILE_FLOATS);
+  float (*ws)[BK][BN] = reinterpret_cast<float (*)[BK][BN]>(tile_smem + group * TILE_FLOATS + 2 * BK * BM);
+  auto meet = [&]() {  // the threads of a group
+    if (GROUPS == 1) __syncthreads();
+    else asm volatile("bar.sync %0, %1;\n" ::"r"(group + 1), "n"(THREADS) : "memory");
+  };
   // A warp is 4 groups of rows by 8 of columns: its vectors of a k are few and shared.
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   constexpr int WARP_COLS = BN / (8 * TN);
   // (a thread's columns: groups of 4, 32 apart, so that 8 lanes read 128 bytes in a row)
   const int mt = ((warp / WARP_COLS) * 4 + (lane >> 3)) * TM, nt = (warp % WARP_COLS) * 8 * TN + (lane & 7) * 4;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int quad = threadIdx.x % QUADS, row = threadIdx.x / QUADS;
+  const int quad = tid % QUADS, row = tid / QUADS;
   auto turn = [](int q) { return (q % 4) * 8 + (q / 4) * 4; };
   constexpr int STEP = THREADS / QUADS;  // rows between a thread's pieces
   float4 xq[XQ], wq[WQ];
+  int k_end = 0;  // of the quarter that is walked (at most K)
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < XQ; ++i) {
       const int r = m0 + row + i * STEP;
-      xq[i] = row_quad(x + (size_t)r * K, r < M, k0 + quad * 4, K, vec);
+      xq[i] = row_quad(x + (size_t)r * K, r < M, k0 + quad * 4, k_end, vec);
     }
 #pragma unroll
     for (int i = 0; i < WQ; ++i) {
       const int r = n0 + row + i * STEP;
-      wq[i] = row_quad(w + (size_t)r * K, r < N, k0 + quad * 4, K, vec);
+      wq[i] = row_quad(w + (size_t)r * K, r < N, k0 + quad * 4, k_end, vec);
     }
   };
   auto put = [&](int buf) {
@@ -95,66 +113,112 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, f
     }
   };
   float2 acc[TM / 2][TN];
+  float* sums = tile_smem + TILE_FLOATS + tid;  // GROUPS 1: this thread's sums so far, THREADS apart
+  const int quarter = f32_quarter(K), parts = GROUPS == 1 ? (K + quarter - 1) / max(quarter, 1) : 4;  // (empty quarters add nothing)
+#pragma unroll 1
+  for (int part = GROUPS == 1 ? 0 : group; part < max(parts, 1); part += GROUPS) {
+    const int k_start = min(part * quarter, K);
+    k_end = min(k_start + quarter, K);
 #pragma unroll
-  for (int i = 0; i < TM / 2; ++i)
+    for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
-  fetch(0);
-  put(0);
-  __syncthreads();
-  for (int k0 = 0, buf = 0; k0 < K; k0 += BK, buf ^= 1) {
-    const bool more = k0 + BK < K;
-    if (more) fetch(k0 + BK);
-    float2 a[2][TM / 2];
-    float b[2][TN];
-    auto read = [&](int s, int k) {
-      const int at = turn(k / 4);
+      for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    if (k_start < k_end) {
+      fetch(k_start);
+      put(0);
+    }
+    meet();
+    for (int k0 = k_start, buf = 0; k0 < k_end; k0 += BK, buf ^= 1) {
+      const bool more = k0 + BK < k_end;
+      if (more) fetch(k0 + BK);
+      float2 a[2][TM / 2];
+      float b[2][TN];
+      auto read = [&](int s, int k) {
+        const int at = turn(k / 4);
 #pragma unroll
-      for (int i = 0; i < TM; i += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(&xs[buf][k][(mt + i) ^ at]);
-        a[s][i / 2] = make_float2(v.x, v.y);
-        a[s][i / 2 + 1] = make_float2(v.z, v.w);
+        for (int i = 0; i < TM; i += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(&xs[buf][k][(mt + i) ^ at]);
+          a[s][i / 2] = make_float2(v.x, v.y);
+          a[s][i / 2 + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int j = 0; j < TN; j += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(&ws[buf][k][(nt + j * 8) ^ at]);
+          b[s][j] = v.x; b[s][j + 1] = v.y; b[s][j + 2] = v.z; b[s][j + 3] = v.w;
+        }
+      };
+      read(0, 0);
+#pragma unroll
+      for (int k = 0; k < BK; ++k) {  // (values beyond the end are zeros on both sides: the chain keeps its value)
+        if (k + 1 < BK) read((k + 1) & 1, k + 1);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          const float2 bb = make_float2(b[k & 1][j], b[k & 1][j]);
+#pragma unroll
+          for (int i = 0; i < TM / 2; ++i) fma_pair(acc[i][j], a[k & 1][i], bb);
+        }
       }
+      if (more) put(buf ^ 1);
+      meet();
+    }
+    if (GROUPS == 1) {
 #pragma unroll
-      for (int j = 0; j < TN; j += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(&ws[buf][k][(nt + j * 8) ^ at]);
-        b[s][j] = v.x; b[s][j + 1] = v.y; b[s][j + 2] = v.z; b[s][j + 3] = v.w;
-      }
-    };
-    read(0, 0);
+      for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {  // (values beyond K are zeros on both sides: the chain keeps its value)
-      if (k + 1 < BK) read((k + 1) & 1, k + 1);
+        for (int j = 0; j < TN; ++j) {
+          float* at = sums + (i * TN + j) * 2 * THREADS;
+          if (part > 0) {
+            acc[i][j].x = at[0] + acc[i][j].x;
+            acc[i][j].y = at[THREADS] + acc[i][j].y;
+          }
+          if (part + 1 < parts) {
+            at[0] = acc[i][j].x;
+            at[THREADS] = acc[i][j].y;
+          }
+        }
+    }
+  }
+  if (GROUPS == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      const int gm = m0 + mt + i;
+      if (gm >= M) break;
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
-        const float2 bb = make_float2(b[k & 1][j], b[k & 1][j]);
-#pragma unroll
-        for (int i = 0; i < TM / 2; ++i) fma_pair(acc[i][j], a[k & 1][i], bb);
+        const int gn = n0 + nt + (j / 4) * 32 + j % 4;
+        if (gn < N) out[(size_t)gm * N + gn] = capped(i & 1 ? acc[i / 2][j].y : acc[i / 2][j].x, cap);
       }
     }
-    if (more) put(buf ^ 1);
-    __syncthreads();
+    return;
   }
+  // The groups' chains meet: [BM][BN] each, in the place of a group's own tiles.
+  float* mine = tile_smem + group * TILE_FLOATS;
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int gm = m0 + mt + i;
-    if (gm >= M) break;
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int gn = n0 + nt + (j / 4) * 32 + j % 4;
-      if (gn < N) out[(size_t)gm * N + gn] = capped(i & 1 ? acc[i / 2][j].y : acc[i / 2][j].x, cap);
+    for (int j = 0; j < TN; j += 4) {
+      const float4 v = i & 1 ? make_float4(acc[i / 2][j].y, acc[i / 2][j + 1].y, acc[i / 2][j + 2].y, acc[i / 2][j + 3].y)
+                             : make_float4(acc[i / 2][j].x, acc[i / 2][j + 1].x, acc[i / 2][j + 2].x, acc[i / 2][j + 3].x);
+      *reinterpret_cast<float4*>(mine + (mt + i) * BN + nt + j * 8) = v;
     }
+  __syncthreads();
+  for (int i = threadIdx.x; i < BM * BN; i += THREADS * GROUPS) {
+    const int gm = m0 + i / BN, gn = n0 + i % BN;
+    if (gm >= M || gn >= N) continue;
+    float sum = tile_smem[i];
+#pragma unroll
+    for (int part = 1; part < GROUPS; ++part) sum += tile_smem[part * TILE_FLOATS + i];
+    out[(size_t)gm * N + gn] = capped(sum, cap);
   }
 }
 
 // ---------------------------------------------------------------------------
 // Up to 16 rows: one output per thread, 128 per block (ROWS x 128 / ROWS).  The weights' rows stream
 // through a ring of asynchronous 16-byte copies (rows of 16-byte multiples only), several blocks per
-// SM; the chain of one output (4 cycles per k) is what is left, so a thread has the vectors of the
-// next 16 k in registers while it multiplies these.
+// SM; a thread walks the four quarters' chains side by side (one chain's FMA waits 4 cycles for the one before).
 // ---------------------------------------------------------------------------
 #define F32_FEW 16        // most rows
-#define F32_FEW_K 128     // k per stage
+#define F32_FEW_K 128     // k per stage: 32 of each quarter
 #define F32_FEW_STAGES 5
 #define F32_FEW_LD (F32_FEW_K + 4)  // a row's start moves on by 4 banks
 
@@ -165,13 +229,14 @@ gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
   constexpr int COLS = 128 / ROWS, STAGE = (COLS + ROWS) * F32_FEW_LD, PIECES = F32_FEW_K / 4;
   extern __shared__ __align__(16) float few_smem[];  // stages of (weights [COLS][LD], x [ROWS][LD])
   const int n0 = blockIdx.x * COLS;
-  const int steps = (K + F32_FEW_K - 1) / F32_FEW_K;
+  const int quarter = f32_quarter(K), steps = quarter / 32;
   // A warp copies a row's 512 bytes at a time.  (Beyond the matrix: 0 bytes read, zeros written.)
   const int piece = (threadIdx.x % PIECES) * 4, first = threadIdx.x / PIECES;
+  const int from_k = piece / 32 * quarter + piece % 32, end_k = min(piece / 32 * quarter + quarter, K);
   auto copy = [&](const float* from, int rows, int count, int step, float* to) {
-    const int k = step * F32_FEW_K + piece;
+    const int k = step * 32 + from_k;
     for (int r = first; r < count; r += 128 / PIECES) {
-      const bool in = r < rows && k < K;
+      const bool in = r < rows && k < end_k;
       const float* src = in ? from + (size_t)r * K + k : from;
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
                        (unsigned)__cvta_generic_to_shared(to + r * F32_FEW_LD + piece)), "l"(src), "r"(in ? 16 : 0));
@@ -188,7 +253,7 @@ gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
     asm volatile("cp.async.commit_group;\n");
   }
   const int m = threadIdx.x / COLS, n = threadIdx.x % COLS;
-  float acc = 0.f;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
   for (int s = 0; s < steps; ++s) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(F32_FEW_STAGES - 2));
     __syncthreads();  // the stage has landed for all; the one read a turn ago is free
@@ -203,32 +268,30 @@ gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
     const float* xr = few_smem + (s % F32_FEW_STAGES) * STAGE + (COLS + m) * F32_FEW_LD;
     if (m < M) {
       float4 a[2][4], b[2][4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        a[0][q] = *reinterpret_cast<const float4*>(xr + 4 * q);
-        b[0][q] = *reinterpret_cast<const float4*>(wr + 4 * q);
-      }
-#pragma unroll
-      for (int k = 0; k < F32_FEW_K; k += 16) {
-        const int at = (k / 16) & 1;
-        if (k + 16 < F32_FEW_K) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            a[at ^ 1][q] = *reinterpret_cast<const float4*>(xr + k + 16 + 4 * q);
-            b[at ^ 1][q] = *reinterpret_cast<const float4*>(wr + k + 16 + 4 * q);
-          }
-        }
+      auto read = [&](int at, int k) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          acc = fmaf(a[at][q].x, b[at][q].x, acc);
-          acc = fmaf(a[at][q].y, b[at][q].y, acc);
-          acc = fmaf(a[at][q].z, b[at][q].z, acc);
-          acc = fmaf(a[at][q].w, b[at][q].w, acc);
+          a[at][q] = *reinterpret_cast<const float4*>(xr + 32 * q + k);
+          b[at][q] = *reinterpret_cast<const float4*>(wr + 32 * q + k);
         }
+      };
+      read(0, 0);
+#pragma unroll
+      for (int k = 0; k < 32; k += 4) {
+        const int at = (k / 4) & 1;
+        if (k + 4 < 32) read(at ^ 1, k + 4);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fmaf(a[at][q].x, b[at][q].x, acc[q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fmaf(a[at][q].y, b[at][q].y, acc[q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fmaf(a[at][q].z, b[at][q].z, acc[q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fmaf(a[at][q].w, b[at][q].w, acc[q]);
       }
     }
   }
-  if (m < M && n0 + n < N) out[(size_t)m * N + n0 + n] = capped(acc, cap);
+  if (m < M && n0 + n < N) out[(size_t)m * N + n0 + n] = capped(((acc[0] + acc[1]) + acc[2]) + acc[3], cap);
 }
 
 template <int ROWS>
@@ -242,12 +305,18 @@ static int launch_f32_few(const float* x, const float* w, float* out, int M, int
   return 0;
 }
 
-template <int BM, int BN, int BK, int TM, int TN>
+template <int BM, int BN, int BK, int TM, int TN, int GROUPS>
 static int launch_f32_tile(const float* x, const float* w, float* out, int M, int N, int K, float cap, int vec,
                            cudaStream_t stream) {
   const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) return -6;
-  sb_launch(gemm_f32_tile_kernel<BM, BN, BK, TM, TN>, grid, (BM / TM) * (BN / TN), 0, stream, x, w, out, M, N, K, cap, vec);
+  constexpr size_t smem = sizeof(float) * (GROUPS * 2 * BK * (BM + BN) + (GROUPS == 1 ? BM * BN : 0));
+  auto kernel = gemm_f32_tile_kernel<BM, BN, BK, TM, TN, GROUPS>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  sb_launch(kernel, grid, (BM / TM) * (BN / TN) * GROUPS, smem, stream, x, w, out, M, N, K, cap, vec);
   SB_LAUNCH_CHECK();
   return 0;
 }
@@ -264,15 +333,40 @@ extern "C" int sb_gemm_f32_tile(int M, int N, int K, int vec) {
   return tiles(64) >= 96 ? 64 : 32;
 }
 
-extern "C" int sb_gemm_f32_nt(const float* x, const float* w, float* out, int M, int N, int K, float cap,
-                              cudaStream_t stream) {
+// Groups of threads a tile of 64 or 32 has for the quarters of k.  Four where the tiles alone leave SMs with too few
+// warps: an SM holds one block of 4 x 128 threads, or four of 128 (us, 1 group against 4, tiles of 64: 256 x 2,048 x
+// 2,048, 128 tiles, 80 and 62, x 8,192 291 and 215; 256 x 3,072 x 2,048, 192, 117 and 113; 44 x 16,384 x 2,048, 256, 117
+// and 113; 600 x 2,048 x 8,192, 320, 631 and 602; 44 x 32,768 x 2,048, 512, 211 and 215; 256 x 16,384 x 2,048, 1,024, 358
+// and 377; 300 x 9,000 x 32 15.2 and 20.5; tiles of 32: 44 x 2,048 x 2,048 70 and 31, x 8,192 253 and 98; 300 x 500 x
+// 1,024 39 and 27; 40 x 200 x 63 10 and 8; 300 x 9,000 x 32 17 and 20).
+extern "C" int sb_gemm_f32_groups(int M, int N, int K, int tile) {
+  const long long tiles = (long long)((N + 63) / 64) * ((M + 63) / 64);
+  return tile <= 64 && K > 32 && (tile == 32 || tiles < 400) ? 4 : 1;
+}
+
+// `tile` and `groups`: 0 for the ones that the sizes choose (others are for tests).
+extern "C" int sb_gemm_f32_nt_as(const float* x, const float* w, float* out, int M, int N, int K, float cap, int tile,
+                                 int groups, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   const int vec = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-  switch (sb_gemm_f32_tile(M, N, K, vec)) {
+  if (tile == 0) tile = sb_gemm_f32_tile(M, N, K, vec);
+  if (tile <= F32_FEW && (!vec || K <= 0 || M > tile)) return -9;
+  if (groups == 0) groups = sb_gemm_f32_groups(M, N, K, tile);
+  switch (tile) {
     case 8: return launch_f32_few<8>(x, w, out, M, N, K, cap, stream);
     case 16: return launch_f32_few<16>(x, w, out, M, N, K, cap, stream);
-    case 128: return launch_f32_tile<128, 128, 16, 16, 8>(x, w, out, M, N, K, cap, vec, stream);
-    case 64: return launch_f32_tile<64, 64, 32, 8, 4>(x, w, out, M, N, K, cap, vec, stream);
-    default: return launch_f32_tile<32, 32, 32, 4, 4>(x, w, out, M, N, K, cap, vec, stream);
+    case 128: return launch_f32_tile<128, 128, 16, 16, 8, 1>(x, w, out, M, N, K, cap, vec, stream);
+    case 64:
+      return groups == 4 ? launch_f32_tile<64, 64, 32, 8, 4, 4>(x, w, out, M, N, K, cap, vec, stream)
+                         : launch_f32_tile<64, 64, 32, 8, 4, 1>(x, w, out, M, N, K, cap, vec, stream);
+    case 32:
+      return groups == 4 ? launch_f32_tile<32, 32, 32, 4, 4, 4>(x, w, out, M, N, K, cap, vec, stream)
+                         : launch_f32_tile<32, 32, 32, 4, 4, 1>(x, w, out, M, N, K, cap, vec, stream);
+    default: return -9;
   }
+}
+
+extern "C" int sb_gemm_f32_nt(const float* x, const float* w, float* out, int M, int N, int K, float cap,
+                              cudaStream_t stream) {
+  return sb_gemm_f32_nt_as(x, w, out, M, N, K, cap, 0, 0, stream);
 }
