@@ -39,6 +39,18 @@ def experts_on_tensor_memory(pairs: int, width: int, hidden: int, gated: bool) -
   return width + hidden >= 1280 or work > 1 << 28
 
 
+def tokens_per_attention_block(tokens: int, requests: int, heads: int) -> int:
+  """How many neighbouring tokens of a request share a block of the general attention kernel (float32 storage,
+  csrc/attention_generic.cu), and with it every key and value that is fetched: as many as leave every SM two blocks, where
+  requests bring that many tokens on average.  us of 1, 2, 4 and 8 (16 heads of 128): 20 tokens 15.0, 15.2, 15.9, 19.7; 64
+  28.6, 20.1, 20.8, 25.5; 130 61.7, 37.9, 28.9, 33.5; 600 687, 322, 261, 213; 3 requests of 20 to 150 93, 57, 52, 51; 8 of
+  9 to 70 62.8, 35.9, 36.5, 38.8."""
+  for together in (8, 4, 2):
+    if tokens >= together * requests and -(-tokens // together) * heads >= 2 * SMS:
+      return together
+  return 1
+
+
 def walks_by_chunks(kind: int, lengths: Sequence[int], heads: int, dim: int, value_dim: int) -> bool:
   """Whether a step's walks through recurrent states go by chunks of tokens (csrc/chunk_walks.cu) or token by token
   (csrc/state_scans.cu): `lengths` new tokens per request, states of dim x value_dim.  One kernel walks all
