@@ -36,7 +36,7 @@ class KernelBuildError(RuntimeError):
 
 
 # Sources that are compiled once per head size (-DSB_HEAD_DIM=N) into libraries of their own.
-PER_HEAD_DIM = ("attention_mma.cu", "attention_tc.cu", "attention_tc_pair.cu")
+PER_HEAD_DIM = ("attention_mma.cu", "attention_rows.cu", "attention_tc.cu", "attention_tc_pair.cu")
 # ... and those of them that also take value heads of another size (-DSB_VALUE_DIM=M).
 PER_TWO_SIZES = ("attention_mma.cu", "attention_tc.cu")
 

@@ -51,6 +51,29 @@ def tokens_per_attention_block(tokens: int, requests: int, heads: int) -> int:
   return 1
 
 
+def attention_cluster(requests: int, kv_heads: int, group: int, dim: int, keys: int) -> int:
+  """Blocks per (request, kv head) of the one-launch decode attention (csrc/attention_rows.cu) for single tokens that
+  see up to `keys` keys, or 0: the split-key kernel (csrc/attention_mma.cu), which streams long contexts better.
+
+  64 blocks where clusters are 8 or 16 wide (more clusters of 8 than two per GPC wait for one another), else up to
+  148, one per SM.  us of a decode step, split keys against one launch (Gemma 2 2B unless said; its requests' keys):
+
+      1 x 1,000 1,530 / 1,470    2 x 1,900 1,577 / 1,551    8 x 900   1,690 / 1,657    24 x 300 2,501 / 2,238
+      1 x 4,000 1,614 / 1,570    2 x 3,900 1,663 / 1,690    8 x 2,000 1,807 / 1,849    24 x 800 2,498 / 2,486
+      1 x 7,000 1,637 / 1,640    4 x 900   1,631 / 1,547    16 x 300  1,986 / 1,851    32 x 700 2,718 / 2,582
+                                 4 x 1,900 1,641 / 1,685    16 x 900  2,119 / 2,068    40 x 900 3,088 / 3,365
+      Gemma 2 9B: 1 x 900 4,201 / 4,070, 8 x 900 4,634 / 4,572
+      heads of 128, four to a kv head: 8 kv heads 1 x 900 487 / 468, 2 x 900 478 / 470, 8 x 900 545 / 558; 4 kv heads
+      1 x 900 594 / 602"""
+  pairs = requests * kv_heads
+  cluster = max((c for c in (1, 2, 4, 8, 16) if pairs * c <= (64 if c >= 8 else 128)), default=0) or int(pairs <= SMS)
+  if not cluster or keys > (256 * cluster if cluster >= 4 else 1024):
+    return 0
+  if dim == 256 and group == 2:
+    return cluster
+  return cluster if dim == 128 and group == 4 and 8 <= pairs <= 16 else 0
+
+
 def walks_by_chunks(kind: int, lengths: Sequence[int], heads: int, dim: int, value_dim: int) -> bool:
   """Whether a step's walks through recurrent states go by chunks of tokens (csrc/chunk_walks.cu) or token by token
   (csrc/state_scans.cu): `lengths` new tokens per request, states of dim x value_dim.  One kernel walks all

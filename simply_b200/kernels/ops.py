@@ -23,7 +23,7 @@ import numpy as np
 import torch
 
 from simply_b200.kernels import build
-from simply_b200.kernels.choices import experts_on_tensor_memory, tokens_per_attention_block, walks_by_chunks
+from simply_b200.kernels.choices import attention_cluster, experts_on_tensor_memory, tokens_per_attention_block, walks_by_chunks
 
 _F32, _BF16 = 0, 1
 _ERRORS = {
@@ -175,6 +175,9 @@ class CudaOps:
     self.direct_library_products = True  # False: through torch.mm
     self._library_workspaces: dict = {}
     self._step_stream = None
+    # Attention of single tokens over few keys in one launch (csrc/attention_rows.cu): None by the step's sizes
+    # (kernels/choices.py), 0 never, 1, 2, 4 or 8: always with so many blocks per request and kv head (tests).
+    self.attention_rows: int | None = None
     # 0: prefill tiles of 64 query rows; 64 or 128 forces a size.
     self.prefill_rows = 0
     # Prefill attention on the tcgen05 tensor cores where the shapes allow (head size a multiple of
@@ -481,6 +484,12 @@ class CudaOps:
         prefill_pair.argtypes = [c_void, c_void, c_void, c_int, c_void, c_void, c_void, c_int, c_int, c_int, c_int,
                                  c_int, c_float, c_int, c_void, c_int, c_void, c_void]
         prefill_pair.restype = c_int
+      rows = None
+      if head_dim in (64, 128, 256) and value_dim == head_dim:
+        rows = getattr(lib, f"sb_attn_rows_{suffix}")
+        rows.argtypes = [c_void, c_void, c_void, c_int, c_void, c_void, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
+                         c_int, c_int, c_void, c_void]
+        rows.restype = c_int
       resident = getattr(lib, f"sb_attn_decode_resident_{suffix}")
       resident.argtypes, resident.restype = [c_int], c_int
       slots = resident(1)
@@ -488,7 +497,7 @@ class CudaOps:
         raise KernelError(f"sb_attn_decode_resident: {_STATUS.get(slots, slots)}")
       self._decode_slots[(head_dim, value_dim)] = slots
       fns = self._attn_fns[(head_dim, value_dim)] = (prefill, decode, make_map, prefill_tc, prefill_pair, prefill_pooled,
-                                                              prefill_biased, prefill_tc_biased)
+                                                              prefill_biased, prefill_tc_biased, rows)
     return fns
 
   def _latent_fn(self, row_dim: int, value_dim: int):
@@ -1166,6 +1175,19 @@ class CudaOps:
       # it takes the shape (no cap beside a distance bias), else the mma.sync tile kernel; not the kernel by pairs.
       options = (_ptr(distance_bias), linear_bias, _ptr(sink), int(key_chunk or 0), keep_first) if special else (None, 0, None, 0, 0)
       kind = dict(key_chunk=key_chunk, value_dim=value_dim, keep_first=keep_first)
+      if fns[8] is not None and not special and ctx.max_q_len == 1 and t == ctx.num_seqs and not self.decode_variant and not self.decode_chunk:
+        cluster = self.attention_rows
+        if cluster is None:
+          cluster = attention_cluster(t, num_kv_heads, group, head_dim, min(ctx.max_kv_len, window or ctx.max_kv_len))
+        if cluster:
+          rc = fns[8](_ptr(q), _ptr(storage), _ptr(block_table), block_table.shape[1], _ptr(ctx.q_start), _ptr(out), t,
+                      num_heads, num_kv_heads, ctx.page_size, storage.shape[0], float(logit_softcap), int(window or 0), cluster,
+                      int(getattr(ctx, "older_keys_settled", False)), _ptr(self.err), self._stream())
+          if rc == 0:
+            self.launches += 1
+            return out
+          if rc != -9:
+            raise KernelError(f"sb_attn_rows: {_STATUS.get(rc, rc)}")
       use_tc = (self._prefill_uses_tcgen05(head_dim, group, ctx.page_size, special or value_dim != head_dim)
                 and (distance_bias is None or not logit_softcap))
       use_pair = (prefill_pair is not None and self._prefill_uses_pairs(head_dim, group, ctx.page_size)

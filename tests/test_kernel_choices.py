@@ -6,7 +6,7 @@ import ctypes
 import pytest
 
 from simply_b200.kernels import build
-from simply_b200.kernels.choices import experts_on_tensor_memory, walks_by_chunks
+from simply_b200.kernels.choices import attention_cluster, experts_on_tensor_memory, walks_by_chunks
 
 
 @pytest.fixture(scope="module")
@@ -107,3 +107,16 @@ def test_walks_that_stay_token_by_token(kind, lengths, dim):
     (64, 16, 2560, 2560, False, (130, 109)), (64, 16, 4096, 3584, False, (219, 178)), (8192, 16, 2048, 2048, False, (913, 199))])
 def test_experts_products_where_they_are_faster(pairs, experts, width, hidden, gated, times):
   assert experts_on_tensor_memory(pairs, width, hidden, gated) == (times[1] < times[0])
+
+
+# requests, kv heads, query heads per kv head, head size, most keys: us of a decode step by split keys and in one launch
+@pytest.mark.parametrize("requests,kv_heads,group,dim,keys,times", [
+    (1, 4, 2, 256, 1024, (1530, 1470)), (1, 4, 2, 256, 4096, (1614, 1570)), (1, 4, 2, 256, 8192, (1637, 1640)),
+    (2, 4, 2, 256, 2048, (1577, 1551)), (2, 4, 2, 256, 4096, (1663, 1690)), (4, 4, 2, 256, 1024, (1631, 1547)),
+    (4, 4, 2, 256, 2048, (1641, 1685)), (8, 4, 2, 256, 1024, (1690, 1657)), (8, 4, 2, 256, 2048, (1807, 1849)),
+    (16, 4, 2, 256, 1024, (2119, 2068)), (24, 4, 2, 256, 1024, (2498, 2486)), (32, 4, 2, 256, 1024, (2718, 2582)),
+    (40, 4, 2, 256, 1024, (3088, 3365)), (1, 8, 2, 256, 1024, (4201, 4070)), (8, 8, 2, 256, 1024, (4634, 4572)),
+    (1, 8, 4, 128, 1024, (487, 468)), (2, 8, 4, 128, 1024, (478, 470)), (8, 8, 4, 128, 1024, (545, 558)),
+    (1, 4, 4, 128, 1024, (594, 602))])
+def test_decode_attention_in_one_launch_where_it_is_faster(requests, kv_heads, group, dim, keys, times):
+  assert bool(attention_cluster(requests, kv_heads, group, dim, keys)) == (times[1] < times[0])
