@@ -144,6 +144,7 @@ class CudaOps:
   # Largest token count the weight-streaming product for a handful of tokens takes, and the largest
   # the one for a serving batch takes (csrc/gemm_skinny_bf16.cu, csrc/gemm_stream_tc.cu).
   skinny_max_rows = 16
+  runs_layers = True  # (`layer_run` may take a model's layers through this table's entry points)
   mid_max_rows = 128
 
   def __init__(self, dtype: torch.dtype = torch.bfloat16, device: str | torch.device = "cuda"):
@@ -201,6 +202,9 @@ class CudaOps:
     self.chunk_walks: bool | None = None
     self._wide_tables: dict[tuple, torch.Tensor] = {}
     self.prefill_single_key_group = False  # True: 64-row tiles with 4 warps instead of 4 x 2 (experiments, tests)
+    # The layers of a step in one call from the host where the model's are all alike (kernels/layer_run.py); False: part
+    # by part (tests).
+    self.layer_runs = True
     # 0: the weight-streaming product picks its warps per block; 4, 8 or 16 forces them (experiments).
     self.skinny_warps = 0
     # False keeps the q, k, v projection and the rotation + cache write as two kernels (tests).
@@ -356,6 +360,8 @@ class CudaOps:
     self.lib.sb_gemm_library_bf16_heads.argtypes = [c_void, c_int, c_int, c_void, c_void, c_int, c_int, c_int, c_int, c_int,
                                                     c_int, ctypes.c_float, c_void, c_ll, c_void]
     self.lib.sb_gemm_library_bf16_heads.restype = c_int
+    self.lib.sb_layer_run.argtypes = [c_void, c_int, c_void, c_void, c_void, c_void, c_void]
+    self.lib.sb_layer_run.restype = c_int
     self.lib.sb_chunk_walk_floats.argtypes = [c_int, c_ll, c_int, c_int, c_int, c_int, c_int]
     self.lib.sb_chunk_walk_floats.restype = c_ll
     self.lib.sb_graph_burst.argtypes = [c_void, c_void, c_void, c_ll, c_int, c_void, c_void, c_ll, c_void]
@@ -375,13 +381,17 @@ class CudaOps:
     instead of once per launch (an engine step is a few hundred launches)."""
     return _HeldStream(self)
 
-  def _library_product(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
-    """out = x . w^T through the matrix-product library with a kept algorithm; False when it
-    has none for this shape."""
+  def _library_workspace(self) -> torch.Tensor:
     stream = self._stream()
     workspace = self._library_workspaces.get(stream.value)
     if workspace is None:  # one per stream: products on different streams may run together
       workspace = self._library_workspaces[stream.value] = torch.empty(32 << 20, dtype=torch.uint8, device=self.device)
+    return workspace
+
+  def _library_product(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """out = x . w^T through the matrix-product library with a kept algorithm; False when it
+    has none for this shape."""
+    stream, workspace = self._stream(), self._library_workspace()
     m, k = x.shape
     rc = self.lib.sb_gemm_library_bf16(_ptr(x), _ptr(w), _ptr(out), m, w.shape[0], k, int(out.dtype == torch.float32),
                                        _ptr(workspace), workspace.numel(), stream)
@@ -396,10 +406,7 @@ class CudaOps:
     call of the matrix-product library (bfloat16); False when it does not take the shape."""
     if x.dtype != torch.bfloat16 or not self.direct_library_products:
       return False
-    stream = self._stream()
-    workspace = self._library_workspaces.get(stream.value)
-    if workspace is None:
-      workspace = self._library_workspaces[stream.value] = torch.empty(32 << 20, dtype=torch.uint8, device=self.device)
+    stream, workspace = self._stream(), self._library_workspace()
     h, n, k = w.shape
     rc = self.lib.sb_gemm_library_bf16_heads(_ptr(x), x.shape[1], x_head, _ptr(w), _ptr(out), out.shape[1], out_head,
                                              x.shape[0], h, n, k, float(alpha), _ptr(workspace), workspace.numel(), stream)
@@ -412,9 +419,13 @@ class CudaOps:
     rc = getattr(self.lib, name)(*args, self._stream())
     self.launches += rc != -9  # -9: the kernel does not take the shape and launched nothing
     if rc != 0 and rc != -9:
-      why = _STATUS.get(rc, f"CUDA error {rc}" if rc > 0 else f"status {rc}")
-      raise KernelError(f"{name}: {why}")
+      self._raise(name, rc)
     return rc
+
+  @staticmethod
+  def _raise(name: str, rc: int) -> None:
+    why = _STATUS.get(rc, f"CUDA error {rc}" if rc > 0 else f"status {rc}")
+    raise KernelError(f"{name}: {why}")
 
   def _new(self, *shape, dtype=None) -> torch.Tensor:
     return torch.empty(shape, dtype=dtype or self.dtype, device=self.device)

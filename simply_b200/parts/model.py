@@ -56,6 +56,7 @@ class DecoderModel:
     self.final_norm = build_part(NORMS, spec.final_norm)
     self.head = build_part(HEADS, spec.head, embedding=self.embedding)
     self.cache_names = spec.cache_names()
+    self._uniform: Any = False  # (not looked at yet; kernels/layer_run.py)
 
   # ---- weights --------------------------------------------------------------
   def tensor_specs(self) -> list[TensorSpec]:
@@ -117,6 +118,21 @@ class DecoderModel:
       raise ValueError(f"layer {layer!r} wants to see {need.window or 'all'} keys of cache {cache!r}, which keeps only {kept}")
 
   # ---- forward --------------------------------------------------------------
+  def _run_layers(self, stream: ResidualStream, ctx: Any, caches: dict[str, Any]) -> bool:
+    """All layers in one call from the host, where the model and the kernel table allow it."""
+    if not getattr(type(ctx.ops), "runs_layers", False):
+      return False
+    from simply_b200.kernels.layer_run import UniformLayers
+    if self._uniform is False:
+      self._uniform = UniformLayers.of(self)
+    if self._uniform is None or not self._uniform.takes(ctx):
+      return False
+    branch = self._uniform.run(stream.h, ctx, caches)
+    if branch is None:
+      return False
+    stream.add(branch, self._uniform.blocks[-1].post_feed_forward, ctx)
+    return True
+
   def forward(self, ctx: Any, caches: dict[str, Any]) -> torch.Tensor | None:
     """Runs the step's tokens; returns float32 logits [R, vocab] at ctx.logit_rows."""
     first = self.embedding.forward(ctx)
@@ -132,7 +148,10 @@ class DecoderModel:
       first, kept = first.clone(), first  # the stream is updated in place: the steps read a copy
     stream = ResidualStream(first)
     layer_outputs = ctx.memo.get("layer_outputs")  # a list: the stream after every layer call (debugging, tests)
-    for call, cache in zip(self.spec.run_order, self.cache_names):
+    calls = list(zip(self.spec.run_order, self.cache_names))
+    if layer_outputs is None and self._run_layers(stream, ctx, caches):
+      calls = []
+    for call, cache in calls:
       if call.add_embedding:
         stream.add_input(again, ctx)
       if call.stream_input is not None:

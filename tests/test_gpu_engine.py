@@ -228,3 +228,31 @@ def test_engine_refuses_without_cuda_kernels(monkeypatch):
   monkeypatch.setattr(torch.cuda, "is_available", lambda: False)
   with pytest.raises(ops_mod.KernelError, match="no CPU path"):
     ops_mod.CudaOps(torch.bfloat16)
+
+
+# rows of each kind of product (16 and fewer, to 32, to 128, more), several requests, single tokens beside prompts, a
+# window; a hidden size that the tcgen05 product takes and one that neither it nor the library does
+@pytest.mark.parametrize("hidden,kv_heads", [(384, 2), (388, 1)])
+@pytest.mark.parametrize("steps", [[[9]], [[16, 1]], [[20, 5], [1, 30]], [[60, 41, 2], [1, 1, 9]], [[150, 3], [1, 140]]])
+def test_layers_in_one_call_give_the_same_bits(monkeypatch, hidden, kv_heads, steps):
+  from simply_b200 import design_bench
+  from simply_b200.config import config_from_dict
+  from simply_b200.kernels.layer_run import UniformLayers
+  d = design_bench.DICTS["gemma2"](dict(width=256, heads=4, kv_heads=kv_heads, dim=64, ff=hidden, vocab=512, layers=3))
+  d.update(sliding_window=48, layer_types=["sliding_attention", "full_attention", "sliding_attention"])
+  ran = []
+  run = UniformLayers.run
+  monkeypatch.setattr(UniformLayers, "run", lambda self, *a: ran.append(run(self, *a)) or ran[-1])
+  got = []
+  for together in (True, False):
+    engine = Engine.from_config(config_from_dict(d), 3, EngineConfig(
+        activation_dtype="bfloat16", page_size=64, batch_size=4, max_seq_len=512, max_num_issue_tokens=512), scale_std=0.1)
+    engine.ops.layer_runs = together
+    slots = [engine.open_request(i) for i in range(max(map(len, steps)))]
+    rng = np.random.default_rng(1)
+    for lengths in steps:
+      got.append(engine.step_raw([StepEntry(s, rng.integers(0, 512, n).tolist(), (n - 1,)) for s, n in zip(slots, lengths)]))
+    engine.ops.check_errors()
+  assert len(ran) == len(steps) and all(b is not None for b in ran)
+  for a, b in zip(got[:len(steps)], got[len(steps):]):
+    assert torch.isfinite(a).all() and torch.equal(a, b)
