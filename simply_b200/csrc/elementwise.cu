@@ -97,8 +97,18 @@ __global__ void residual_norm_kernel(float* __restrict__ h, const T* __restrict_
   if (one_chunk) {
     // The row fits one 16-byte chunk per thread: every load is issued before the first sum, so
     // the kernel pays one memory latency instead of one per pass.  Same arithmetic as below.
-    const int i = threadIdx.x * N;
+    // The block's two sums meet at one barrier each: every warp adds the warps' parts up for itself, in block_sum's
+    // order (three barriers a sum took 2 to 3 % longer: 2,048 rows of 2,304 14.6 and 14.4 us, 3,001 of 3,584 35.4 and
+    // 34.6, 1 row 1.99 and 1.91; two rows per block, for more loads in flight, 16.4 and 32.4: the registers then leave
+    // an SM half the blocks).
+    const int i = threadIdx.x * N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const bool on = i < width;
+    auto sum_of_block = [&](float x, float* place) {
+      x = warp_sum(x);
+      if (lane == 0) place[warp] = x;
+      __syncthreads();
+      return warp_sum(lane < nwarps ? place[lane] : 0.f);
+    };
     float b[N], b2[TWO ? N : 1], v[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) b[k] = v[k] = 0.f;
@@ -118,7 +128,7 @@ __global__ void residual_norm_kernel(float* __restrict__ h, const T* __restrict_
         float ss = 0.f;
 #pragma unroll
         for (int k = 0; k < N; ++k) ss += b[k] * b[k];
-        ss = block_sum(ss, scratch);
+        ss = sum_of_block(ss, row);
         rstd_b = 1.0f / sqrtf(ss / (float)width + eps_post);
       }
 #pragma unroll
@@ -137,7 +147,7 @@ __global__ void residual_norm_kernel(float* __restrict__ h, const T* __restrict_
       float ss = 0.f;
 #pragma unroll
       for (int k = 0; k < N; ++k) ss += v[k] * v[k];
-      ss = block_sum(ss, scratch);
+      ss = sum_of_block(ss, row + 32);
       const float rstd = 1.0f / sqrtf(ss / (float)width + eps_pre);
       if (on) {
         float o[N];
@@ -255,11 +265,13 @@ extern "C" int sb_residual_norm(float* h, const void* branch, const void* branch
   if (width % vec == 0 && width / vec <= 1024) threads = ((width / vec + 31) / 32) * 32;
   if (threads < 64) threads = 64;
   if (branch2 != nullptr && branch == nullptr) return -3;
+  // (one vector per thread: the warps' parts of two sums; else the row and block_sum's scratch)
+  const size_t bytes = width % vec == 0 && width <= threads * vec ? 64 * sizeof(float) : smem;
 #define SB_RESIDUAL(T_, TWO_)                                                                                    \
   do {                                                                                                           \
     auto k = residual_norm_kernel<T_, TWO_>;                                                                     \
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
-    sb_launch(k, num_rows, threads, smem, stream, h, (const T_*)branch, (const T_*)branch2, w_post, post_f32,    \
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);     \
+    sb_launch(k, num_rows, threads, bytes, stream, h, (const T_*)branch, (const T_*)branch2, w_post, post_f32,   \
               eps_post, post_plus_one, w_pre, pre_f32, eps_pre, pre_plus_one, rows, (T_*)y, width, num_rows_total, \
               err);                                                                                              \
   } while (0)
