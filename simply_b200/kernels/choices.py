@@ -74,6 +74,20 @@ def attention_cluster(requests: int, kv_heads: int, group: int, dim: int, keys: 
   return cluster if dim == 128 and group == 4 and 8 <= pairs <= 16 else 0
 
 
+def few_rows_join_tiles(keys: Sequence[int], kv_heads: int) -> bool:
+  """Whether the requests of a step that bring only a few tokens beside prompts (`keys`: how many each sees) are tiles of
+  the prompts' attention kernel too (csrc/attention_tc_pair.cu), in place of a split-key launch and its merge behind
+  it.  A tile takes one of 74 pairs of blocks 7.5 us and 7 us per 1,000 keys.  us of a step of Gemma 2 2B, split keys
+  and tiles (requests of one token x keys, the prompt, the tiles' estimated us):
+
+      8 x 200,  100  2,673 / 2,295   3.8      16 x 600, 400  3,898 / 3,541  10.1      39 x 300, 100  3,213 / 3,305  20.2
+      8 x 600,  400  3,579 / 3,141   5.1      39 x 100, 100  3,013 / 3,034  17.3      39 x 300, 400  4,042 / 4,051  20.2
+      16 x 200, 100  2,872 / 2,464   7.7      39 x 100, 400  3,899 / 3,753  17.3      39 x 600, 100  3,492 / 3,590  24.7
+
+  prompts of 3 to 1,500 tokens together 14,001 / 13,230; of 2 and 600 4,247 / 3,982."""
+  return sum(7.5 + 0.007 * k for k in keys) * kv_heads / 74 < 16.0
+
+
 def walks_by_chunks(kind: int, lengths: Sequence[int], heads: int, dim: int, value_dim: int) -> bool:
   """Whether a step's walks through recurrent states go by chunks of tokens (csrc/chunk_walks.cu) or token by token
   (csrc/state_scans.cu): `lengths` new tokens per request, states of dim x value_dim.  One kernel walks all

@@ -23,7 +23,7 @@ import numpy as np
 import torch
 
 from simply_b200.kernels import build
-from simply_b200.kernels.choices import attention_cluster, experts_on_tensor_memory, tokens_per_attention_block, walks_by_chunks
+from simply_b200.kernels.choices import attention_cluster, experts_on_tensor_memory, few_rows_join_tiles, tokens_per_attention_block, walks_by_chunks
 
 _F32, _BF16 = 0, 1
 _ERRORS = {
@@ -179,6 +179,8 @@ class CudaOps:
     # Attention of single tokens over few keys in one launch (csrc/attention_rows.cu): None by the step's sizes
     # (kernels/choices.py), 0 never, 1, 2, 4 or 8: always with so many blocks per request and kv head (tests).
     self.attention_rows: int | None = None
+    # Requests of a few new tokens beside prompts may be tiles of the prompts' kernel (False: tests).
+    self.few_rows_in_tiles = True
     # 0: prefill tiles of 64 query rows; 64 or 128 forces a size.
     self.prefill_rows = 0
     # Prefill attention on the tcgen05 tensor cores where the shapes allow (head size a multiple of
@@ -681,6 +683,10 @@ class CudaOps:
     cu_q, q_start = ctx.host["cu_q"], ctx.host["q_start"].astype(np.int64)
     q_len = np.diff(cu_q).astype(np.int64)
     small = (q_len * group <= 16) & (not all_tiles)  # all_tiles: the tile kernel takes every sequence
+    if force_rows == 256 and self.few_rows_in_tiles and small.any() and not small.all():
+      keys = q_start + q_len - self.lowest_keys(q_start, window, key_chunk)
+      if few_rows_join_tiles(keys[small].tolist(), num_kv_heads):
+        small[:] = False
     # Tiles of 64 query rows (finer grains balance better over the SMs than tiles of 128).
     rows_per_tile = force_rows or self.prefill_rows or 64
     tokens_per_tile = rows_per_tile // group

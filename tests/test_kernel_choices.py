@@ -6,7 +6,7 @@ import ctypes
 import pytest
 
 from simply_b200.kernels import build
-from simply_b200.kernels.choices import attention_cluster, experts_on_tensor_memory, walks_by_chunks
+from simply_b200.kernels.choices import attention_cluster, experts_on_tensor_memory, few_rows_join_tiles, walks_by_chunks
 
 
 @pytest.fixture(scope="module")
@@ -120,3 +120,11 @@ def test_experts_products_where_they_are_faster(pairs, experts, width, hidden, g
     (1, 4, 4, 128, 1024, (594, 602))])
 def test_decode_attention_in_one_launch_where_it_is_faster(requests, kv_heads, group, dim, keys, times):
   assert bool(attention_cluster(requests, kv_heads, group, dim, keys)) == (times[1] < times[0])
+
+
+# requests of one token, their keys: us of a step with them on split keys and as tiles beside a prompt
+@pytest.mark.parametrize("requests,keys,times", [
+    (8, 200, (2673, 2295)), (8, 600, (3579, 3141)), (16, 200, (2872, 2464)), (16, 600, (3898, 3541)), (39, 100, (3013, 3034)),
+    (39, 300, (3213, 3305)), (39, 600, (3492, 3590)), (1, 3, (14001, 13230))])
+def test_few_rows_are_tiles_where_that_is_faster(requests, keys, times):
+  assert few_rows_join_tiles([keys] * requests, 4) == (times[1] < times[0])
