@@ -139,9 +139,8 @@ class UniformLayers:
     layers = np.array(rows, dtype=np.int64)
     y, q, attended, mixed = new(t, width), new(t, heads, dim), new(t, heads * dim), new(t, width)
     z, down = new(t, hidden), new(t, width)
-    qkv, gate_up = new(t, (heads + 2 * kv_heads) * dim), new(t, 2 * hidden) if t < o.gated_tc_min_rows or hidden % 128 else None
-    if gate_up is None and o.gated_tc_min_rows <= 0:
-      gate_up = new(t, 2 * hidden)
+    # (what a product stores that no fused kernel takes; steps are short here, so all of it is always there)
+    qkv, gate_up = new(t, (heads + 2 * kv_heads) * dim), new(t, 2 * hidden)
     mid = o.mid_rows if o.mid_rows_kernel else dict.fromkeys(o.mid_rows, 0)
     workspace = o._library_workspace()
     step = _Step(

@@ -231,14 +231,14 @@ def test_engine_refuses_without_cuda_kernels(monkeypatch):
 
 
 # rows of each kind of product (16 and fewer, to 32, to 128, more), several requests, single tokens beside prompts, a
-# window; a hidden size that the tcgen05 product takes and one that neither it nor the library does
-@pytest.mark.parametrize("hidden,kv_heads", [(384, 2), (388, 1)])
+# window; sizes that the tcgen05 product takes, and a hidden size and a width that neither it nor the library does
+@pytest.mark.parametrize("width,hidden,kv_heads", [(256, 384, 2), (256, 388, 1), (260, 384, 2)])
 @pytest.mark.parametrize("steps", [[[9]], [[16, 1]], [[20, 5], [1, 30]], [[60, 41, 2], [1, 1, 9]], [[150, 3], [1, 140]]])
-def test_layers_in_one_call_give_the_same_bits(monkeypatch, hidden, kv_heads, steps):
+def test_layers_in_one_call_give_the_same_bits(monkeypatch, width, hidden, kv_heads, steps):
   from simply_b200 import design_bench
   from simply_b200.config import config_from_dict
   from simply_b200.kernels.layer_run import UniformLayers
-  d = design_bench.DICTS["gemma2"](dict(width=256, heads=4, kv_heads=kv_heads, dim=64, ff=hidden, vocab=512, layers=3))
+  d = design_bench.DICTS["gemma2"](dict(width=width, heads=4, kv_heads=kv_heads, dim=64, ff=hidden, vocab=512, layers=3))
   d.update(sliding_window=48, layer_types=["sliding_attention", "full_attention", "sliding_attention"])
   ran = []
   run = UniformLayers.run
