@@ -93,7 +93,7 @@ class AttentionGraphPlan:
   def __init__(self, ops: "CudaOps", window: int | None, group: int, num_kv_heads: int, head_dim: int,
                batch: int, bucket: int, max_burst: int, page_size: int, key_chunk: int | None = None,
                value_dim: int | None = None, keep_first: int = 0):
-    self.key = ops._plan_key(window, group, num_kv_heads, head_dim, page_size, key_chunk, value_dim, keep_first)
+    self.key = ops._plan_key(window, group, num_kv_heads, head_dim, key_chunk, value_dim, keep_first)
     self.window, self.key_chunk, self.group, self.batch = window, key_chunk, group, batch
     self.keep_first = keep_first
     # Most keys a sequence of this bucket sees in such a layer during a burst.
@@ -627,20 +627,13 @@ class CudaOps:
     return (self.prefill_pairs and self._prefill_uses_tcgen05(head_dim, group, page_size)
             and head_dim in (128, 256) and page_size >= 64)
 
-  def _prefill_rows(self, head_dim: int, group: int, page_size: int) -> int:
-    """Query rows of a prefill work item: 256 for a pair of blocks, 128 for the tcgen05 kernel, else the mma.sync tile."""
-    if self._prefill_uses_pairs(head_dim, group, page_size):
-      return 256
-    if self._prefill_uses_tcgen05(head_dim, group, page_size):
-      return 128
-    return self.prefill_rows or 64
-
-  def _plan_key(self, window: int | None, group: int, num_kv_heads: int, head_dim: int, page_size: int,
-                key_chunk: int | None = None, value_dim: int | None = None, keep_first: int = 0) -> tuple:
-    """Where a step keeps the work lists of one kind of attention layer in `ctx.memo`.  Layers
-    share lists only if everything the lists are cut for agrees: the window, the group, the
-    number of kv heads and the head size (they set the chunk length) and the rows of a prefill tile."""
-    key = ("attention_plan", window, group, num_kv_heads, head_dim, self._prefill_rows(head_dim, group, page_size))
+  @staticmethod
+  def _plan_key(window: int | None, group: int, num_kv_heads: int, head_dim: int, key_chunk: int | None = None,
+                value_dim: int | None = None, keep_first: int = 0) -> tuple:
+    """Where a decode graph keeps the static list of one kind of attention layer in `ctx.memo`: everything that the
+    split-key kernel's list is cut for (the window, the group, the number of kv heads and the head size, which set
+    the chunk length).  Single tokens have no tiles, so layers whose prompts go to different kernels share it."""
+    key = ("attention_plan", window, group, num_kv_heads, head_dim)
     other_values = value_dim if value_dim != head_dim else None
     if keep_first:
       return key + (key_chunk, other_values, keep_first)
@@ -664,19 +657,26 @@ class CudaOps:
     group = num_heads // num_kv_heads
     if value_dim != head_dim or not window or not self._uses_tensor_core_attention(head_dim, group):
       return None
-    return PooledAttentionGraphPlan(self._plan_key(window, group, num_kv_heads, head_dim, page_size) + ("pooled", pool), batch)
+    return PooledAttentionGraphPlan(self._plan_key(window, group, num_kv_heads, head_dim) + ("pooled", pool), batch)
 
   def _attention_plan(self, ctx: Any, window: int | None, group: int, force_rows: int = 0,
                       num_kv_heads: int = 1, head_dim: int = 0, tag: tuple = (), all_tiles: bool = False,
                       key_chunk: int | None = None, value_dim: int | None = None, keep_first: int = 0) -> dict:
-    """Work lists of the two tensor-core kernels for this step, per kind of layer (`_plan_key`).
+    """Work lists of the two tensor-core kernels for this step, per kind of layer (`_plan_key`) and kernel for its
+    prompts: `force_rows` 256 the tcgen05 kernel by pairs, 128 the one by single blocks, 0 the mma.sync kernel.  Their
+    tiles differ, and with them which requests the split-key kernel is left with: layers share a list only if
+    their prompts go to the same kernel.
 
     Sequences with at most 16 query rows per kv head (one or a few new tokens) go to the
     split-key kernel: their keys are cut into chunks at multiples of `chunk` of the
     absolute position, one work item per chunk.  The others are cut into tiles of
     64 // group or 128 // group tokens for the prefill kernel, heaviest tile first.
     """
-    key = self._plan_key(window, group, num_kv_heads, head_dim, ctx.page_size, key_chunk, value_dim, keep_first) + tag
+    key = self._plan_key(window, group, num_kv_heads, head_dim, key_chunk, value_dim, keep_first)
+    plan = ctx.memo.get(key)  # (a decode graph brings its static list)
+    if plan is not None:
+      return plan
+    key += ("prompts", force_rows) + tag
     plan = ctx.memo.get(key)
     if plan is not None:
       return plan
@@ -729,7 +729,7 @@ class CudaOps:
     n_pre, n_dec = prefill_items.size, decode_items.size
     plan = dict(
         num_prefill=len(prefill_items), num_decode=len(decode_items), chunk=chunk, rows_per_tile=rows_per_tile,
-        item_width=prefill_items.shape[1], rows_max=int((q_len[dec] * group).max()) if len(dec) else 0,
+        rows_max=int((q_len[dec] * group).max()) if len(dec) else 0,
         prefill_items=dev[:n_pre], decode_items=dev[n_pre:n_pre + n_dec],
         split_start=dev[n_pre + n_dec:n_pre + n_dec + num_seqs], split_count=dev[n_pre + n_dec + num_seqs:])
     ctx.memo[key] = plan
@@ -1170,7 +1170,7 @@ class CudaOps:
       if not tensor_cores:
         general()
         return out
-      key = self._plan_key(window, group, num_kv_heads, head_dim, ctx.page_size) + ("pooled", pool_len)
+      key = self._plan_key(window, group, num_kv_heads, head_dim) + ("pooled", pool_len)
       plan = ctx.memo.get(key)  # (a decode graph brings its static list)
       if plan is None:
         plan = self._attention_plan(ctx, window, group, 0, num_kv_heads, head_dim, tag=("pooled", pool_len),
@@ -1220,11 +1220,8 @@ class CudaOps:
         if rc:
           raise KernelError(f"sb_attn_prefill_pair: {_STATUS.get(rc, rc)}")
       elif plan["num_prefill"] and use_tc and special:
-        tiles = plan
-        if plan["rows_per_tile"] != 128 or plan.get("item_width") != 3:  # (a list cut for another kernel)
-          tiles = self._attention_plan(ctx, window, group, 128, num_kv_heads, head_dim, tag=("rows", 128), **kind)
-        rc = fns[7](*common, _ptr(out), t, *sizes, _ptr(tiles["prefill_items"]),
-                                              tiles["num_prefill"], *options, _ptr(self.err), self._stream())
+        rc = fns[7](*common, _ptr(out), t, *sizes, _ptr(plan["prefill_items"]), plan["num_prefill"], *options,
+                    _ptr(self.err), self._stream())
         self.launches += 1
         if rc:
           raise KernelError(f"sb_attn_prefill_tc_biased: {_STATUS.get(rc, rc)}")
@@ -1235,11 +1232,8 @@ class CudaOps:
         if rc:
           raise KernelError(f"sb_attn_prefill_tc: {_STATUS.get(rc, rc)}")
       elif plan["num_prefill"] and special:
-        tiles = plan
-        if plan.get("item_width", 2) != 2:  # (a list cut for the tcgen05 kernels, made by a layer without a bias)
-          tiles = self._attention_plan(ctx, window, group, 64, num_kv_heads, head_dim, tag=("rows", 64), **kind)
         rc = fns[6](
-            *common, _ptr(out), *sizes, _ptr(tiles["prefill_items"]), tiles["num_prefill"], tiles["rows_per_tile"],
+            *common, _ptr(out), *sizes, _ptr(plan["prefill_items"]), plan["num_prefill"], plan["rows_per_tile"],
             int(self.prefill_single_key_group), *options, _ptr(self.err), self._stream())
         self.launches += 1
         if rc:

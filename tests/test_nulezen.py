@@ -121,6 +121,22 @@ def test_long_prompts_pages_of_64_and_head_sizes_of_the_tensor_core_kernels(dtyp
   engine.ops.check_errors()
 
 
+@pytest.mark.gpu
+def test_few_tokens_beside_prompts_in_layers_with_and_without_the_bias():
+  """Heads of 128 over pages of 64, one window for both kinds of layer: prompts, requests of a few tokens and
+  decoded tokens share steps."""
+  sizes = dict(heads=8, kv_heads=4, dim=128, vdim=128, window=300, scale=0.07)
+  cfg_dict = nx.config([nx.rotated(dims=64, base=5000.0, **sizes), nx.biased(**sizes), nx.rotated(dims=64, base=5000.0, **sizes)],
+                       [nx.dense(ff=256)] * 3, width=128, vocab=300)
+  cfg, t = nx.weights(cfg_dict, seed=3, matrix_std=0.1)
+  engine = nx.build_engine(cfg, t, "bfloat16", "cuda", None, page_size=64, slots=4, max_seq_len=512)
+  requests = [tokens_for(cfg_dict, n, 10 + i) for i, n in enumerate([330, 60, 400, 24, 210])]
+  got = nx.run_mixed(engine, requests, seed=4, max_live=4, portions=(1, 3, 120, 180))
+  for i, (g, toks) in enumerate(zip(got, requests)):
+    nx.check_close(g, plain.forward(cfg_dict, nx.as_numpy(t), toks), "bfloat16", f"request {i} in a mixed batch")
+  engine.ops.check_errors()
+
+
 @pytest.mark.parametrize("where", WHERE)
 def test_many_query_heads_per_kv_head(where):
   """32 and 12 query heads per kv head: a single token's rows no longer fit the split-key kernel's
