@@ -3,7 +3,10 @@
 // tiles of 32 that start at a multiple of 32 of the absolute key position, tile number i
 // by warp i mod 4, and the warps' parts are merged in warp order, so a token's result is
 // the same whatever else the step holds.  A prompt's tokens come 2, 4 or 8 to a block, which share every
-// key and value that is fetched; each of them adds up in the order it has alone.
+// key and value that is fetched; each of them adds up in the order it has alone.  A block's tokens belong to one
+// request: where requests meet inside a group of 2, 4 or 8 tokens, each has a block of its own, and a token alone in its
+// block is walked as blocks of one token walk it (a group walked request by request, 16 heads of 128, us by blocks
+// of one token, so, and now: 31 requests of one token and 4,000 keys beside a prompt of 600 1,452, 6,550, 1,368, 7 of 2,000 beside 256 439, 2,296, 232).
 //
 //   s = q . k                 (q is already rotated and scaled)
 //   s = cap * tanh(s / cap)   if cap > 0          simply/model_lib.py:621-626
@@ -29,6 +32,8 @@
 // This is the true 32-bit path's attention and the fallback of the bfloat16
 // path for shapes its tensor-core kernels refuse.
 #include <float.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -139,12 +144,15 @@ __device__ __forceinline__ void gen_tile(const KT* kr, const KT* vr, unsigned se
   }
 }
 
-// R > 1: without pooled blocks, distances and kept first keys.
+// R > 1: without pooled blocks, distances and kept first keys.  Its blocks: (a request but the first, query head), for the
+// request's first tokens where those lie inside a group of R tokens, then (group of R tokens, query head), for the
+// first request of the group: every run of one request's tokens within a group once.
 template <typename T, int R, int DPL>
 __global__ void __launch_bounds__(GEN_WARPS * 32)
 paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ cache,
                                const int* __restrict__ block_table, int max_pages,
                                const int* __restrict__ token_seq, const int* __restrict__ positions,
+                               const int* __restrict__ cu_q, int num_seqs,
                                T* __restrict__ out, int num_tokens, int num_q_heads, int num_kv_heads,
                                int head_dim, int v_dim, int page_size, int num_pages, float cap, int window,
                                const T* __restrict__ pool, const int* __restrict__ pool_table,
@@ -155,39 +163,48 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ ca
   const float r2 = distance != nullptr && !linear ? distance[num_q_heads + blockIdx.x % num_q_heads] : 0.f;
   pdl_wait_block();
   pdl_launch_dependents();
-  // R * head_dim floats of q, then per query and warp its running maximum, sum and v_dim partial results
-  extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long item = blockIdx.x;
-  const int t_first = (int)(item / num_q_heads) * R, n = (int)(item % num_q_heads);
+  const int n = blockIdx.x % num_q_heads;
   const int m = n / (num_q_heads / num_kv_heads);
-  float* qs = smem;
-  float* part = smem + R * head_dim;
-  // Tokens of one sequence at a time (a block's tokens may belong to several).
-  for (int t = t_first; t < min(t_first + R, num_tokens);) {
-    const int b = token_seq[t];
-    int count = 1;
-    while (count < R && t + count < min(t_first + R, num_tokens) && token_seq[t + count] == b) ++count;
-    int pos[R], lo[R];
+  int t = blockIdx.x / num_q_heads, count = 1;
+  if (R > 1) {
+    const int others = num_seqs - 1, s = t + 1;
+    if (t < others) {
+      t = cu_q[s];
+      if (t < 0 || t >= num_tokens || t % R == 0 || token_seq[t] != s) return;  // (a group's first token, or no new token)
+    } else {
+      t = (t - others) * R;
+    }
+    const int end = min(t / R * R + R, num_tokens);
+    while (t + count < end && token_seq[t + count] == token_seq[t]) ++count;
+  }
+  const int b = token_seq[t];
+  // The block's `count` tokens from t on, at most N; N * head_dim floats of q, then per query and warp its running
+  // maximum, sum and v_dim partial results.
+  extern __shared__ __align__(16) float smem[];
+  auto attend = [&](auto most) {
+    constexpr int N = decltype(most)::value;
+    float* qs = smem;
+    float* part = smem + N * head_dim;
+    int pos[N], lo[N];
     int pos_all = 0, lo_all = 0;  // the highest and the lowest key that one of them sees
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < N; ++r) {
       pos[r] = r < count ? positions[t + r] : -1;
       lo[r] = window > 0 ? max(pos[r] - window + 1, 0) : chunk > 0 ? max(pos[r], 0) / chunk * chunk : 0;
       if (r == 0 || (r < count && pos[r] > pos_all)) pos_all = pos[r];
       if (r == 0 || (r < count && lo[r] < lo_all)) lo_all = lo[r];
     }
-    __syncthreads();  // (the run before has been stored)
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < N; ++r) {
       const T* qp = q + ((size_t)(t + min(r, count - 1)) * num_q_heads + n) * head_dim;
       for (int d = threadIdx.x; d < head_dim; d += blockDim.x) qs[r * head_dim + d] = to_f32<T>(qp[d]);
     }
     __syncthreads();
 
-    float m_run[R], l_run[R], acc[R][DPL];
+    float m_run[N], l_run[N], acc[N][DPL];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < N; ++r) {
       m_run[r] = -0.5f * FLT_MAX;
       l_run[r] = 0.f;
 #pragma unroll
@@ -214,7 +231,7 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ ca
             vr = pool + page * page_stride + (size_t)num_kv_heads * entries * head_dim + row * v_dim;
           }
         }
-        gen_tile<T, R, DPL>(kr, vr, kr != nullptr, qs, head_dim, v_dim, cap, 0.f, lane, m_run, l_run, acc);
+        gen_tile<T, N, DPL>(kr, vr, kr != nullptr, qs, head_dim, v_dim, cap, 0.f, lane, m_run, l_run, acc);
       }
     }
 
@@ -230,7 +247,7 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ ca
       const T* vr = nullptr;
       unsigned sees = 0;
 #pragma unroll
-      for (int r = 0; r < R; ++r) sees |= (j >= lo[r] || j < keep) && j <= pos[r] ? 1u << r : 0u;
+      for (int r = 0; r < N; ++r) sees |= (j >= lo[r] || j < keep) && j <= pos[r] ? 1u << r : 0u;
       if (sees) {
         const long long page = block_table[(size_t)b * max_pages + j / page_size];
         if (page < 0 || page >= num_pages) {
@@ -245,12 +262,12 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ ca
       float minus = 0.f;
       if (R == 1 && distance != nullptr && j <= pos[0])
         minus = r1 * (linear ? (float)(pos[0] - j) : log1pf(r2 * (float)(pos[0] - j)));
-      gen_tile<T, R, DPL>(kr, vr, sees, qs, head_dim, v_dim, cap, minus, lane, m_run, l_run, acc);
+      gen_tile<T, N, DPL>(kr, vr, sees, qs, head_dim, v_dim, cap, minus, lane, m_run, l_run, acc);
     }
     // The warps' parts meet in warp order (the same order whatever the step holds).
     const int stride = v_dim + 2;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < N; ++r) {
       float* mine = part + (size_t)(r * GEN_WARPS + warp) * stride;
       if (lane == 0) {
         mine[0] = m_run[r];
@@ -285,7 +302,18 @@ paged_attention_generic_kernel(const T* __restrict__ q, const T* __restrict__ ca
         op[d] = from_f32<T>(sum * inv);
       }
     }
-    t += count;
+  };
+  if (R == 1) {
+    // (One turn.  Written as a loop: as straight code nvcc 12.9 fetches the values one by one here, 600 tokens of 16
+    // heads of 128 864 us in place of 688, in bfloat16 1,057 in place of 562.)
+    for (const int end = min(t + 1, num_tokens); t < end; ++t) {
+      __syncthreads();
+      attend(std::integral_constant<int, 1>{});
+    }
+  } else if (count == 1) {
+    attend(std::integral_constant<int, 1>{});
+  } else {
+    attend(std::integral_constant<int, R>{});
   }
 }
 
@@ -296,7 +324,8 @@ extern "C" int sb_paged_attention_general(const void* q, int dtype, const void* 
                                           int window, const void* pool, const int* pool_table,
                                           int pool_max_pages, int pool_len, int pool_pages, int tied,
                                           const float* sink, const float* distance, int linear, int chunk,
-                                          int keep, int together, int* err, cudaStream_t stream) {
+                                          int keep, const int* cu_q, int num_seqs, int together, int* err,
+                                          cudaStream_t stream) {
   if (num_tokens == 0) return 0;
   if (distance != nullptr && pool != nullptr) return -13;
   if (chunk > 0 && (pool != nullptr || window > 0)) return -13;
@@ -308,7 +337,7 @@ extern "C" int sb_paged_attention_general(const void* q, int dtype, const void* 
   if (pool != nullptr || distance != nullptr || keep > 0 || dtype != SB_DTYPE_F32 || v_dim > 256) together = 1;
   if (v_dim > 128) together = min(together, 4);
   const int rows = together >= 8 ? 8 : together >= 4 ? 4 : together >= 2 ? 2 : 1;
-  const long long items = (long long)((num_tokens + rows - 1) / rows) * num_q_heads;
+  const long long items = ((long long)((num_tokens + rows - 1) / rows) + (rows > 1 ? num_seqs - 1 : 0)) * num_q_heads;
   if (items > 0x7fffffffLL) return -6;
   const unsigned blocks = (unsigned)items;
   const size_t smem = rows * ((size_t)head_dim + (size_t)GEN_WARPS * (v_dim + 2)) * sizeof(float);
@@ -320,8 +349,8 @@ extern "C" int sb_paged_attention_general(const void* q, int dtype, const void* 
       if (e != cudaSuccess) return (int)e;                                                                              \
     }                                                                                                                   \
     sb_launch(kernel, blocks, GEN_WARPS * 32, smem, stream, (const T_*)q, (const T_*)cache, block_table, max_pages,     \
-              token_seq, positions, (T_*)out, num_tokens, num_q_heads, num_kv_heads, head_dim, v_dim, page_size,        \
-              num_pages, cap, window, (const T_*)pool, pool_table, pool_max_pages, pool_len, pool_pages, tied, sink,    \
+              token_seq, positions, cu_q, num_seqs, (T_*)out, num_tokens, num_q_heads, num_kv_heads, head_dim, v_dim,    \
+              page_size, num_pages, cap, window, (const T_*)pool, pool_table, pool_max_pages, pool_len, pool_pages, tied, sink,    \
               distance, linear, chunk, keep, err);                                                                      \
   } while (0)
   if (dtype != SB_DTYPE_F32) SB_GENERIC(bf16, 1, GEN_MAX_DPL);
@@ -339,8 +368,9 @@ extern "C" int sb_paged_attention_generic(const void* q, int dtype, const void* 
                                           int max_pages, const int* token_seq, const int* positions,
                                           void* out, int num_tokens, int num_q_heads, int num_kv_heads,
                                           int head_dim, int page_size, int num_pages, float cap, int window,
-                                          int together, int* err, cudaStream_t stream) {
+                                          const int* cu_q, int num_seqs, int together, int* err, cudaStream_t stream) {
   return sb_paged_attention_general(q, dtype, cache, block_table, max_pages, token_seq, positions, out, num_tokens,
                                     num_q_heads, num_kv_heads, head_dim, head_dim, page_size, num_pages, cap,
-                                    window, nullptr, nullptr, 0, 0, 0, 0, nullptr, nullptr, 0, 0, 0, together, err, stream);
+                                    window, nullptr, nullptr, 0, 0, 0, 0, nullptr, nullptr, 0, 0, 0, cu_q,
+                                    num_seqs, together, err, stream);
 }

@@ -42,9 +42,10 @@ def experts_on_tensor_memory(pairs: int, width: int, hidden: int, gated: bool) -
 def tokens_per_attention_block(tokens: int, requests: int, heads: int) -> int:
   """How many neighbouring tokens of a request share a block of the general attention kernel (float32 storage,
   csrc/attention_generic.cu), and with it every key and value that is fetched: as many as leave every SM two blocks, where
-  requests bring that many tokens on average.  us of 1, 2, 4 and 8 (16 heads of 128): 20 tokens 15.0, 15.2, 15.9, 19.7; 64
-  28.6, 20.1, 20.8, 25.5; 130 61.7, 37.9, 28.9, 33.5; 600 687, 322, 261, 213; 3 requests of 20 to 150 93, 57, 52, 51; 8 of
-  9 to 70 62.8, 35.9, 36.5, 38.8."""
+  requests bring that many tokens on average (a request's last tokens and single ones have blocks of their own).  us of 1,
+  2, 4 and 8 (16 heads of 128): 20 tokens 11.4, 11.3, 13.0, 15.7; 64 27.6, 16.9, 16.7, 20.4; 130 58.5, 34.2, 30.8, 31.0;
+  600 694, 329, 244, 212; 3 requests of 20 to 150 88, 47, 38, 38; 8 of 9 to 70 70.1, 33.4, 31.6, 35.8; 7 of one token and
+  2,000 keys beside a prompt of 256 439, 360, 287, 232; 31 of one and 4,000 beside 600 1,482, 1,047, 1,009, 1,368."""
   for together in (8, 4, 2):
     if tokens >= together * requests and -(-tokens // together) * heads >= 2 * SMS:
       return together

@@ -270,10 +270,11 @@ class CudaOps:
         "sb_qkv_rope_skinny": [c_void, c_void, c_int, c_int, c_void, c_void, c_float, c_void, c_void, c_void, c_int,
                                c_void, c_void, c_int, c_int, c_int, c_int, c_int, c_void, c_int, c_void],
         "sb_paged_attention_generic": [c_void, c_int, c_void, c_void, c_int, c_void, c_void, c_void, c_int,
-                                       c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void, c_void],
+                                       c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void, c_int, c_int, c_void, c_void],
         "sb_paged_attention_general": [c_void, c_int, c_void, c_void, c_int, c_void, c_void, c_void, c_int,
                                        c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void, c_void,
-                                       c_int, c_int, c_int, c_int, c_void, c_void, c_int, c_int, c_int, c_int, c_void, c_void],
+                                       c_int, c_int, c_int, c_int, c_void, c_void, c_int, c_int, c_int, c_void, c_int, c_int, c_void,
+                                       c_void],
         "sb_norm_of_sum": [c_void, c_void, c_int, c_float, c_void, c_int, c_float, c_int, c_void, c_int, c_int, c_void],
         "sb_conv_headnorm_store": [c_void, c_int, c_int, c_void, c_int, c_void, c_void, c_int, c_int, c_int, c_void,
                                    c_void, c_float, c_float, c_void, c_int, c_int, c_void, c_void, c_void, c_int, c_void,
@@ -1140,7 +1141,7 @@ class CudaOps:
                    block_table.shape[1], _ptr(ctx.token_seq), _ptr(ctx.positions), _ptr(out), t, num_heads,
                    num_kv_heads, head_dim, value_dim, ctx.page_size, storage.shape[0], float(logit_softcap),
                    int(window or 0), *pool_args, int(values_in_keys), _ptr(sink), _ptr(distance_bias), linear_bias,
-                   int(key_chunk or 0), keep_first, together, _ptr(self.err))
+                   int(key_chunk or 0), keep_first, _ptr(ctx.cu_q), ctx.num_seqs, together, _ptr(self.err))
 
       # bfloat16 with key size = value size: the tensor-core tile kernel (mma.sync tiles of 64 rows,
       # the block entries in tiles of their own ahead of the tokens) for prompt portions and single
@@ -1261,7 +1262,7 @@ class CudaOps:
     self._call("sb_paged_attention_generic", _ptr(q), _code(q), _ptr(storage), _ptr(block_table),
                block_table.shape[1], _ptr(ctx.token_seq), _ptr(ctx.positions), _ptr(out), t, num_heads,
                num_kv_heads, head_dim, ctx.page_size, storage.shape[0], float(logit_softcap),
-               int(window or 0), together, _ptr(self.err))
+               int(window or 0), _ptr(ctx.cu_q), ctx.num_seqs, together, _ptr(self.err))
     return out
 
   # ---- attention with normed queries and keys ---------------------------------

@@ -6,7 +6,7 @@ import ctypes
 import pytest
 
 from simply_b200.kernels import build
-from simply_b200.kernels.choices import attention_cluster, experts_on_tensor_memory, few_rows_join_tiles, walks_by_chunks
+from simply_b200.kernels.choices import attention_cluster, experts_on_tensor_memory, few_rows_join_tiles, tokens_per_attention_block, walks_by_chunks
 
 
 @pytest.fixture(scope="module")
@@ -128,3 +128,15 @@ def test_decode_attention_in_one_launch_where_it_is_faster(requests, kv_heads, g
     (39, 300, (3213, 3305)), (39, 600, (3492, 3590)), (1, 3, (14001, 13230))])
 def test_few_rows_are_tiles_where_that_is_faster(requests, keys, times):
   assert few_rows_join_tiles([keys] * requests, 4) == (times[1] < times[0])
+
+
+# tokens, requests: us of float32 attention (16 heads of 128) with 1, 2, 4 and 8 tokens per block
+@pytest.mark.parametrize("tokens,requests,times", [
+    (20, 1, (11.4, 11.3, 13.0, 15.7)), (64, 1, (27.6, 16.9, 16.7, 20.4)), (130, 1, (58.5, 34.2, 30.8, 31.0)),
+    (256, 1, (162, 82, 70, 69)), (600, 1, (694, 329, 244, 212)), (247, 3, (87.6, 47.2, 38.0, 38.4)),
+    (283, 8, (70.1, 33.4, 31.6, 35.8)), (263, 8, (439, 360, 287, 232)), (615, 16, (808, 421, 332, 322)),
+    (631, 32, (1482, 1047, 1009, 1368))])
+def test_tokens_per_block_of_float32_attention(tokens, requests, times):
+  got = times[(1, 2, 4, 8).index(tokens_per_attention_block(tokens, requests, 16))]
+  # (the last: single tokens with 6 times the prompt's keys, whose blocks then are few to an SM)
+  assert got <= (1.15 if requests < 32 else 1.4) * min(times)
