@@ -75,18 +75,37 @@ def attention_cluster(requests: int, kv_heads: int, group: int, dim: int, keys: 
   return cluster if dim == 128 and group == 4 and 8 <= pairs <= 16 else 0
 
 
-def few_rows_join_tiles(keys: Sequence[int], kv_heads: int) -> bool:
+def few_rows_join_tiles(keys: Sequence[int], prompt_keys: Sequence[int], kv_heads: int, rows: int, key_bytes: int) -> bool:
   """Whether the requests of a step that bring only a few tokens beside prompts (`keys`: how many each sees) are tiles of
   the prompts' attention kernel too (csrc/attention_tc_pair.cu), in place of a split-key launch and its merge behind
-  it.  A tile takes one of 74 pairs of blocks 7.5 us and 7 us per 1,000 keys.  us of a step of Gemma 2 2B, split keys
-  and tiles (requests of one token x keys, the prompt, the tiles' estimated us):
+  it.  `prompt_keys`: the keys of each of the prompts' tiles; `rows`: the step's tokens times query heads; `key_bytes`: of a
+  key and its value.
 
-      8 x 200,  100  2,673 / 2,295   3.8      16 x 600, 400  3,898 / 3,541  10.1      39 x 300, 100  3,213 / 3,305  20.2
-      8 x 600,  400  3,579 / 3,141   5.1      39 x 100, 100  3,013 / 3,034  17.3      39 x 300, 400  4,042 / 4,051  20.2
-      16 x 200, 100  2,872 / 2,464   7.7      39 x 100, 400  3,899 / 3,753  17.3      39 x 600, 100  3,492 / 3,590  24.7
+  A tile is walked from end to end by one of 74 pairs of blocks: 9 us and 14.5 us per 1,000 keys (19 with a prompt's
+  full rows), for heads of 128 and 256 alike.  So a lone request of many keys is the longest walk of the step unless a
+  prompt's is longer, and many requests take several rounds of pairs.  The split keys take 8 us, 1 us per 1,000 rows (the
+  merge looks at each) and what their keys need at 5 TB/s.  us of the attention of a layer, split keys and tiles (requests
+  of one token x keys; 8 and 4 heads of 256 | 32 and 8 of 128):
 
-  prompts of 3 to 1,500 tokens together 14,001 / 13,230; of 2 and 600 4,247 / 3,982."""
-  return sum(7.5 + 0.007 * k for k in keys) * kv_heads / 74 < 16.0
+                  beside 60 tokens         beside 400                beside 4,000
+      1 x 1,000   32, 29  | 26, 30         38, 29  | 42, 30          142, 95  | 396, 255
+      1 x 8,000   47, 128 | 35, 120        46, 126 | 50, 121         151, 135 | 405, 267
+      4 x 4,000   42, 74  | 40, 72         50, 74  | 56, 71          154, 112 | 409, 283
+      16 x 300    34, 24  | 32, 35         40, 34  | 48, 45          144, 109 | 401, 280
+      32 x 600    44, 47  | 46, 77         52, 48  | 63, 82          156, 131 | 417, 317
+
+  A step of Gemma 2 2B: 1 x 7,000 beside 60 2,680 and 4,357, beside 5,000 21,547 and 20,042; 8 x 300 beside 400 3,900
+  and 3,284; prompts of 3 to 1,500 tokens together 14,001 and 13,230."""
+  pairs = 74
+
+  def rounds(costs: list[float]) -> float:  # when the last pair is done
+    costs.sort(reverse=True)
+    tiles = len(costs) * kv_heads  # (of j * pairs + 1 tiles one pair has j + 1)
+    return max([sum(costs) * kv_heads / pairs] + [(j + 1) * costs[pairs * j // kv_heads] for j in range(-(-tiles // pairs))])
+
+  prompts = [9 + 0.019 * k for k in prompt_keys]
+  split = 8 + 0.001 * rows + sum(keys) * kv_heads * key_bytes / 5e6
+  return rounds(prompts + [9 + 0.0145 * k for k in keys]) < rounds(prompts) + split
 
 
 def walks_by_chunks(kind: int, lengths: Sequence[int], heads: int, dim: int, value_dim: int) -> bool:

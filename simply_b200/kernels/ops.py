@@ -684,21 +684,28 @@ class CudaOps:
     cu_q, q_start = ctx.host["cu_q"], ctx.host["q_start"].astype(np.int64)
     q_len = np.diff(cu_q).astype(np.int64)
     small = (q_len * group <= 16) & (not all_tiles)  # all_tiles: the tile kernel takes every sequence
-    if force_rows == 256 and self.few_rows_in_tiles and small.any() and not small.all():
-      keys = q_start + q_len - self.lowest_keys(q_start, window, key_chunk)
-      if few_rows_join_tiles(keys[small].tolist(), num_kv_heads):
-        small[:] = False
     # Tiles of 64 query rows (finer grains balance better over the SMs than tiles of 128).
     rows_per_tile = force_rows or self.prefill_rows or 64
     tokens_per_tile = rows_per_tile // group
     num_seqs = len(q_len)
-    pre = []
-    for b in np.nonzero(~small)[0]:
-      for i0 in range(0, int(q_len[b]), tokens_per_tile):
-        last = int(q_start[b]) + min(i0 + tokens_per_tile, int(q_len[b]))
-        at = int(q_start[b]) + i0
-        first = max(at - window + 1, 0) if window else at // key_chunk * key_chunk if key_chunk else 0
-        pre.append((last - first + min(keep_first, first), int(b), i0))
+
+    def tiles(seqs: np.ndarray) -> list:
+      got = []
+      for b in seqs:
+        for i0 in range(0, int(q_len[b]), tokens_per_tile):
+          last = int(q_start[b]) + min(i0 + tokens_per_tile, int(q_len[b]))
+          at = int(q_start[b]) + i0
+          first = max(at - window + 1, 0) if window else at // key_chunk * key_chunk if key_chunk else 0
+          got.append((last - first + min(keep_first, first), int(b), i0))
+      return got
+
+    pre = tiles(np.nonzero(~small)[0])
+    if force_rows == 256 and self.few_rows_in_tiles and pre and small.any():
+      few = tiles(np.nonzero(small)[0])
+      if few_rows_join_tiles([t[0] for t in few], [t[0] for t in pre], num_kv_heads, int(cu_q[-1]) * num_kv_heads * group,
+                             4 * head_dim):
+        pre += few
+        small[:] = False
     pre.sort(key=lambda x: -x[0])
     if force_rows in (128, 256):
       # The tcgen05 kernels' blocks, one per (tile of queries, kv head), longest walk first over all

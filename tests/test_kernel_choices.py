@@ -122,12 +122,25 @@ def test_decode_attention_in_one_launch_where_it_is_faster(requests, kv_heads, g
   assert bool(attention_cluster(requests, kv_heads, group, dim, keys)) == (times[1] < times[0])
 
 
-# requests of one token, their keys: us of a step with them on split keys and as tiles beside a prompt
-@pytest.mark.parametrize("requests,keys,times", [
-    (8, 200, (2673, 2295)), (8, 600, (3579, 3141)), (16, 200, (2872, 2464)), (16, 600, (3898, 3541)), (39, 100, (3013, 3034)),
-    (39, 300, (3213, 3305)), (39, 600, (3492, 3590)), (1, 3, (14001, 13230))])
-def test_few_rows_are_tiles_where_that_is_faster(requests, keys, times):
-  assert few_rows_join_tiles([keys] * requests, 4) == (times[1] < times[0])
+# heads, kv heads, head size, the prompt, requests of one token and their keys: us of a layer's attention by split keys and
+# as tiles
+@pytest.mark.parametrize("heads,kv_heads,dim,prompt,requests,keys,times", [
+    (8, 4, 256, 60, 1, 200, (29.7, 18.4)), (8, 4, 256, 60, 1, 2000, (31.7, 45.9)), (8, 4, 256, 60, 1, 8000, (47.0, 127.8)),
+    (8, 4, 256, 60, 4, 4000, (42.0, 73.7)), (8, 4, 256, 60, 8, 300, (31.6, 21.5)), (8, 4, 256, 60, 32, 600, (43.9, 47.1)),
+    (8, 4, 256, 400, 1, 1000, (37.9, 28.7)), (8, 4, 256, 400, 1, 4000, (39.9, 71.7)), (8, 4, 256, 400, 16, 300, (39.9, 33.8)),
+    (8, 4, 256, 1500, 1, 4000, (70.7, 72.7)), (8, 4, 256, 1500, 1, 8000, (76.8, 127.0)), (8, 4, 256, 1500, 32, 600, (82.9, 65.5)),
+    (8, 4, 256, 4000, 1, 8000, (150.5, 135.2)), (8, 4, 256, 4000, 32, 600, (155.6, 131.1)),
+    (16, 8, 256, 60, 8, 1500, (48.1, 43.7)), (16, 8, 256, 60, 32, 100, (35.9, 54.2)), (16, 8, 256, 400, 32, 100, (46.1, 54.3)),
+    (16, 8, 256, 400, 32, 600, (70.7, 85.0)), (16, 8, 256, 1500, 1, 8000, (97.0, 131.9)), (16, 8, 256, 1500, 32, 600, (113.7, 109.6)),
+    (32, 8, 128, 60, 1, 8000, (34.9, 119.9)), (32, 8, 128, 60, 8, 300, (27.6, 20.5)), (32, 8, 128, 400, 8, 1500, (52.2, 47.1)),
+    (32, 8, 128, 400, 32, 600, (62.5, 82.1)), (32, 8, 128, 1500, 1, 4000, (126.0, 71.7)), (32, 8, 128, 4000, 32, 600, (416.8, 317.4)),
+    (16, 4, 128, 60, 1, 1000, (25.6, 28.7)), (16, 4, 128, 60, 16, 1000, (31.7, 30.7)), (16, 4, 128, 400, 1, 8000, (41.7, 120.8)),
+    (16, 4, 128, 1500, 1, 4000, (76.8, 70.5)), (16, 4, 128, 4000, 1, 8000, (216.1, 140.3))])
+def test_few_rows_are_tiles_where_that_is_faster(heads, kv_heads, dim, prompt, requests, keys, times):
+  tile = 256 // (heads // kv_heads)
+  prompts = [min(i + tile, prompt) for i in range(0, prompt, tile)]
+  joined = few_rows_join_tiles([keys + 1] * requests, prompts, kv_heads, (prompt + requests) * heads, 4 * dim)
+  assert times[joined] <= 1.04 * min(times)
 
 
 # tokens, requests: us of float32 attention (16 heads of 128) with 1, 2, 4 and 8 tokens per block
