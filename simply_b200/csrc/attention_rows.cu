@@ -18,6 +18,8 @@
 // (1,000 keys 1,514: the second tile's trip is not hidden), 8 warps a block (1,517), 3 stages (as 2).
 #include <math.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "tma_mbar.cuh"
 
@@ -37,7 +39,7 @@ constexpr int WARPS = 16;
 constexpr int LD = 4;      // copies per lane and tile, of keys and of values
 constexpr int STAGES = 2;  // tiles on their way per warp: 128 KB a block
 constexpr int RING_BYTES = STAGES * 2 * LD * WARPS * 32 * 16;
-[[maybe_unused]] constexpr int MAX_CLUSTER = 16;
+constexpr int MAX_CLUSTER = 16;
 [[maybe_unused]] constexpr float LOG2E = 1.4426950408889634f;
 
 struct RowsParams {
@@ -319,19 +321,51 @@ __global__ void __launch_bounds__(WARPS * 32, 1) attn_rows_kernel(const RowsPara
   sbx::cluster_sync_all();  // (nobody leaves while its numbers may be read)
 }
 
+// How many clusters of this size the current device holds at once: 0 where it has no room for one (blocks of 128 KB
+// and 16 warps need an SM each, all in one GPC) or cannot say.  Asked once per device and size.
+template <int G>
+int clusters_held(int cluster) {
+  constexpr int DEVICES = 64;
+  static std::atomic<int> known[DEVICES][MAX_CLUSTER + 1];  // one more than the number; 0: not asked yet
+  int device = -1;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (device < DEVICES) {
+    const int held = known[device][cluster].load(std::memory_order_relaxed);
+    if (held > 0) return held - 1;
+  }
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(cluster);
+  config.blockDim = dim3(WARPS * 32);
+  config.dynamicSmemBytes = RING_BYTES;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = cluster;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  int held = 0;
+  if (cudaFuncSetAttribute(attn_rows_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES) != cudaSuccess ||
+      (cluster > 8 &&
+       cudaFuncSetAttribute(attn_rows_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&held, attn_rows_kernel<G>, &config) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (device < DEVICES) known[device][cluster].store(held + 1, std::memory_order_relaxed);
+  return held;
+}
+
 template <int G>
 int launch(const RowsParams& p, int blocks, int cluster, cudaStream_t stream) {
+  if (clusters_held<G>(cluster) < 1) return -9;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(blocks);
   config.blockDim = dim3(WARPS * 32);
   config.dynamicSmemBytes = RING_BYTES;
-  static const cudaError_t attributed =
-      cudaFuncSetAttribute(attn_rows_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES);
-  if (attributed != cudaSuccess) return (int)attributed;
-  if (cluster > 8) {
-    static const cudaError_t large = cudaFuncSetAttribute(attn_rows_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (large != cudaSuccess) return (int)large;
-  }
   config.stream = stream;
   cudaLaunchAttribute attribute[2];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
@@ -350,9 +384,11 @@ int launch(const RowsParams& p, int blocks, int cluster, cudaStream_t stream) {
 
 }  // namespace
 
+static bool cluster_size(int cluster) { return cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8 || cluster == 16; }
+
 // One token for each of `batch` requests, row b of q and out; cluster: blocks per (request, kv head), 1, 2, 4, 8 or 16.
 // Returns -9 for what it does not take (other head sizes, groups other than 2 and 4, pages of no
-// power of two or shorter than a tile of keys).
+// power of two or shorter than a tile of keys, clusters that the device has no room for).
 extern "C" int SB_FN(sb_attn_rows)(const void* q, const void* cache, const int* block_table, int max_pages, const int* q_start,
                                    void* out, int batch, int num_q_heads, int num_kv_heads, int page_size, int num_pages,
                                    float cap, int window, int cluster, int older_keys_settled, int* err, cudaStream_t stream) {
@@ -361,7 +397,7 @@ extern "C" int SB_FN(sb_attn_rows)(const void* q, const void* cache, const int* 
   if (num_kv_heads <= 0 || num_q_heads % num_kv_heads) return -8;
   const int group = num_q_heads / num_kv_heads;
   if ((group != 2 && group != 4) || page_size <= 0 || page_size < LD * 256 / DH || (page_size & (page_size - 1)) ||
-      (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8 && cluster != 16) || ((uintptr_t)q & 15) || ((uintptr_t)cache & 15))
+      !cluster_size(cluster) || ((uintptr_t)q & 15) || ((uintptr_t)cache & 15))
     return -9;
   int shift = 0;
   while (1 << shift < page_size) ++shift;

@@ -2,6 +2,9 @@
 plain functions of sizes, so no GPU is needed."""
 
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -120,6 +123,16 @@ def test_experts_products_where_they_are_faster(pairs, experts, width, hidden, g
     (1, 4, 4, 128, 1024, (594, 602))])
 def test_decode_attention_in_one_launch_where_it_is_faster(requests, kv_heads, group, dim, keys, times):
   assert bool(attention_cluster(requests, kv_heads, group, dim, keys)) == (times[1] < times[0])
+
+
+def test_decode_attention_in_one_launch_is_refused_where_no_cluster_fits():
+  """A device that holds no cluster of the size that is asked for (here: no device at all) is a shape the kernel does not
+  take, status -9, and the split keys take the step."""
+  call = ("import ctypes; from simply_b200.kernels import build; lib = ctypes.CDLL(build.build_attention(256, verbose=False)); "
+          "p = ctypes.c_void_p(1 << 20); z = ctypes.c_void_p(0); f = lib.sb_attn_rows_hd256; "
+          "print([f(p, p, p, 8, p, p, 1, 8, 4, 64, 8, ctypes.c_float(0), 0, c, 0, p, z) for c in (1, 2, 4, 8, 16)])")
+  done = subprocess.run([sys.executable, "-c", call], env={**os.environ, "CUDA_VISIBLE_DEVICES": ""}, capture_output=True, text=True)
+  assert done.stdout.split("\n")[-2] == str([-9] * 5), done.stdout + done.stderr
 
 
 # heads, kv heads, head size, the prompt, requests of one token and their keys: us of a layer's attention by split keys and
