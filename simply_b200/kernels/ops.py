@@ -177,7 +177,7 @@ class CudaOps:
     self._library_workspaces: dict = {}
     self._step_stream = None
     # Attention of single tokens over few keys in one launch (csrc/attention_rows.cu): None by the step's sizes
-    # (kernels/choices.py), 0 never, 1, 2, 4 or 8: always with so many blocks per request and kv head (tests).
+    # (kernels/choices.py), 0 never, 1, 2, 4, 8 or 16: always with so many blocks per request and kv head (tests).
     self.attention_rows: int | None = None
     # Requests of a few new tokens beside prompts may be tiles of the prompts' kernel (False: tests).
     self.few_rows_in_tiles = True
@@ -499,7 +499,7 @@ class CudaOps:
                                  c_int, c_float, c_int, c_void, c_int, c_void, c_void]
         prefill_pair.restype = c_int
       rows = None
-      if head_dim in (64, 128, 256) and value_dim == head_dim:
+      if head_dim in (128, 256) and value_dim == head_dim:
         rows = getattr(lib, f"sb_attn_rows_{suffix}")
         rows.argtypes = [c_void, c_void, c_void, c_int, c_void, c_void, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
                          c_int, c_int, c_void, c_void]
