@@ -44,6 +44,10 @@ class _Step(ctypes.Structure):
 # 3,300 in all 13,982 and 14,025; 9B, 300 tokens 10,953 and 10,941, 3,001 50,544 and 50,746).
 MOST_OPERATIONS = 1e11
 
+# What the one call stands for: a kernel table on which one of these has been replaced goes part by part.
+STANDS_FOR = frozenset(("residual_norm", "project_rotate_store", "rope_and_cache_write", "paged_attention", "linear",
+                        "gated_linear", "gated_activation", "_call"))
+
 
 class UniformLayers:
 
@@ -83,7 +87,8 @@ class UniformLayers:
     o = ctx.ops
     return (o.layer_runs and ctx.num_tokens * self.operations_per_token <= MOST_OPERATIONS and o.dtype == torch.bfloat16 and ctx.max_q_len > 1 and o.tensor_core_attention
             and o.fused_qkv_rope and o.direct_library_products and o.gated_tc_pairs
-            and not (o.skinny_warps or o.gated_tc_blocks or o.mid_split or o.mid_stages or o.decode_variant))
+            and not (o.skinny_warps or o.gated_tc_blocks or o.mid_split or o.mid_stages or o.decode_variant)
+            and STANDS_FOR.isdisjoint(vars(o)))
 
   def run(self, h: torch.Tensor, ctx: Any, caches: dict[str, Any]):
     """Runs the layers over the stream h (float32, updated in place); returns the last layer's branch, which is

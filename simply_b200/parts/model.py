@@ -120,7 +120,7 @@ class DecoderModel:
   # ---- forward --------------------------------------------------------------
   def _run_layers(self, stream: ResidualStream, ctx: Any, caches: dict[str, Any]) -> bool:
     """All layers in one call from the host, where the model and the kernel table allow it."""
-    if not getattr(type(ctx.ops), "runs_layers", False):
+    if not vars(type(ctx.ops)).get("runs_layers", False):  # (not inherited: a table's own entry points are to be called)
       return False
     from simply_b200.kernels.layer_run import UniformLayers
     if self._uniform is False:

@@ -1,0 +1,32 @@
+"""When a model's layers go to the device in one call (kernels/layer_run.py).  No GPU is needed."""
+
+import types
+
+import pytest
+
+from simply_b200.config import preset
+from simply_b200.kernels import layer_run
+from simply_b200.kernels.ops import CudaOps
+from simply_b200.parts.model import DecoderModel
+
+
+class OwnProducts(CudaOps):
+
+  def linear(self, x, w):
+    return super().linear(x, w)
+
+
+@pytest.mark.parametrize("table,replaced,want", [(CudaOps, None, True), (OwnProducts, None, False), (CudaOps, "linear", False),
+                                                 (CudaOps, "paged_attention", False)])
+def test_a_table_with_entry_points_of_its_own_goes_part_by_part(monkeypatch, table, replaced, want):
+  ops = object.__new__(table)
+  ops.dtype = layer_run.torch.bfloat16
+  ops.layer_runs = ops.tensor_core_attention = ops.fused_qkv_rope = ops.direct_library_products = ops.gated_tc_pairs = True
+  ops.skinny_warps = ops.gated_tc_blocks = ops.mid_split = ops.mid_stages = ops.decode_variant = 0
+  if replaced:
+    setattr(ops, replaced, lambda *a, **kw: None)
+  ran = []
+  monkeypatch.setattr(layer_run.UniformLayers, "run", lambda self, *a: ran.append(a))
+  model = DecoderModel(preset("gemma2-2b").model_spec())
+  model._run_layers(types.SimpleNamespace(h=None), types.SimpleNamespace(ops=ops, num_tokens=20, max_q_len=20), {})
+  assert bool(ran) == want
