@@ -61,6 +61,11 @@ struct SbRunStep {
   float limit, q_scale, cap, eps;
 };
 
+// Bytes of a layer, an attention and a step, for the host's mirrors.
+extern "C" int sb_layer_run_bytes(int which) {
+  return (int)(which == 0 ? sizeof(SbRunLayer) : which == 1 ? sizeof(SbRunAttention) : sizeof(SbRunStep));
+}
+
 // A product that the library has no algorithm for: the caller runs it (layer, 0 qkv, 1 output, 2 gate and up, 3 down).
 typedef int (*SbOtherProduct)(int, int);
 

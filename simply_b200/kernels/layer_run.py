@@ -38,6 +38,8 @@ class _Step(ctypes.Structure):
               + [(n, _F) for n in ("limit", "q_scale", "cap", "eps")])
 
 
+LAYER_WORDS = 16  # numbers of 64 bits per layer
+
 # Operations of a layer's products from which the parts issue a step's launches as fast as the device runs them (about
 # 90 us a layer).  Beyond it nothing is gained, and a queue that is always full was measured to cost 0.3 to 0.5 % (us,
 # parts and one call, Gemma 2 2B: 13 tokens 2,478 and 1,660, 90 3,507 and 2,215, 2,048 8,715 and 8,763; 7 prompts of
@@ -54,6 +56,7 @@ class UniformLayers:
   def __init__(self, blocks: list, names: list[str]):
     self.blocks, self.names = blocks, names
     m, f = blocks[0].mixer, blocks[0].feed_forward
+    self.head_dim, self.group = m.head_dim, m.num_heads // m.num_kv_heads
     # 2 operations per weight and token: q, k, v, output, gate, up, down
     self.operations_per_token = 2.0 * m.width * (2 * (m.num_heads + m.num_kv_heads) * m.head_dim + 3 * f.hidden)
 
@@ -85,10 +88,11 @@ class UniformLayers:
   def takes(self, ctx: Any) -> bool:
     """Whether this step goes this way (its table's options at their defaults)."""
     o = ctx.ops
-    return (o.layer_runs and ctx.num_tokens * self.operations_per_token <= MOST_OPERATIONS and o.dtype == torch.bfloat16 and ctx.max_q_len > 1 and o.tensor_core_attention
-            and o.fused_qkv_rope and o.direct_library_products and o.gated_tc_pairs
+    return (o.layer_runs and ctx.num_tokens * self.operations_per_token <= MOST_OPERATIONS and o.dtype == torch.bfloat16
+            and ctx.max_q_len > 1 and o.fused_qkv_rope and o.direct_library_products and o.gated_tc_pairs
             and not (o.skinny_warps or o.gated_tc_blocks or o.mid_split or o.mid_stages or o.decode_variant)
-            and STANDS_FOR.isdisjoint(vars(o)))
+            and STANDS_FOR.isdisjoint(vars(o)) and o._uses_tensor_core_attention(self.head_dim, self.group)
+            and o._prefill_uses_tcgen05(self.head_dim, self.group, ctx.page_size))
 
   def run(self, h: torch.Tensor, ctx: Any, caches: dict[str, Any]):
     """Runs the layers over the stream h (float32, updated in place); returns the last layer's branch, which is
@@ -97,9 +101,7 @@ class UniformLayers:
     first = self.blocks[0]
     m, f = first.mixer, first.feed_forward
     heads, kv_heads, dim, width, hidden = m.num_heads, m.num_kv_heads, m.head_dim, m.width, f.hidden
-    group = heads // kv_heads
-    if not o._uses_tensor_core_attention(dim, group) or not o._prefill_uses_tcgen05(dim, group, ctx.page_size):
-      return None
+    group = self.group
     scales = first.pre_mixer.weight.dtype
     for b in self.blocks:
       products = (b.mixer.qkv_weight, b.mixer.o_proj.weight, b.feed_forward.gate_up_weight, b.feed_forward.down_proj.weight)
@@ -142,6 +144,7 @@ class UniformLayers:
                    at(cos), at(sin), (tensor_map.value or 0) if tensor_map is not None else 0, cache.storage.shape[0],
                    table.shape[1], kinds[b.mixer.window]))
     layers = np.array(rows, dtype=np.int64)
+    assert layers.shape[1] == LAYER_WORDS
     y, q, attended, mixed = new(t, width), new(t, heads, dim), new(t, heads * dim), new(t, width)
     z, down = new(t, hidden), new(t, width)
     # (what a product stores that no fused kernel takes; steps are short here, so all of it is always there)

@@ -1,10 +1,17 @@
 """Generation through the public entry point on the GPU, against the plain model."""
 
+import dataclasses
+import types
+
 import numpy as np
 import pytest
 import torch
 
-from simply_b200 import Engine, EngineConfig, SamplingParams, StepEntry
+from simply_b200 import Engine, EngineConfig, SamplingParams, StepEntry, design_bench
+from simply_b200.config import PartSpec, config_from_dict
+from simply_b200.kernels.layer_run import UniformLayers
+from simply_b200.parts.model import DecoderModel
+from simply_b200.weights import random_tensors
 from tests.plain.gemma2_plain import PlainGemma2
 from tests.tiny_models import write_tiny
 from tests.tolerances import assert_logits_close
@@ -235,9 +242,6 @@ def test_engine_refuses_without_cuda_kernels(monkeypatch):
 @pytest.mark.parametrize("width,hidden,kv_heads", [(256, 384, 2), (256, 388, 1), (260, 384, 2)])
 @pytest.mark.parametrize("steps", [[[9]], [[16, 1]], [[20, 5], [1, 30]], [[60, 41, 2], [1, 1, 9]], [[150, 3], [1, 140]]])
 def test_layers_in_one_call_give_the_same_bits(monkeypatch, width, hidden, kv_heads, steps):
-  from simply_b200 import design_bench
-  from simply_b200.config import config_from_dict
-  from simply_b200.kernels.layer_run import UniformLayers
   d = design_bench.DICTS["gemma2"](dict(width=width, heads=4, kv_heads=kv_heads, dim=64, ff=hidden, vocab=512, layers=3))
   d.update(sliding_window=48, layer_types=["sliding_attention", "full_attention", "sliding_attention"])
   ran = []
@@ -256,3 +260,51 @@ def test_layers_in_one_call_give_the_same_bits(monkeypatch, width, hidden, kv_he
   assert len(ran) == len(steps) and all(b is not None for b in ran)
   for a, b in zip(got[:len(steps)], got[len(steps):]):
     assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+def _rearranged(spec, block="sandwich_norm", activation="gelu_tanh", limit=0.0, position=True):
+  """The same layers as blocks of another kind, with another activation, without rotations."""
+  layers = []
+  for layer in spec.layers:
+    mixer, ff = dict(layer.mixer.params), dict(layer.feed_forward.params, activation=activation, limit=limit)
+    if not position:
+      mixer["position"] = PartSpec("none")
+    layers.append(dataclasses.replace(
+        layer, block=dataclasses.replace(layer.block, kind=block), mixer=dataclasses.replace(layer.mixer, params=mixer),
+        feed_forward=dataclasses.replace(layer.feed_forward, params=ff)))
+  return dataclasses.replace(spec, layers=tuple(layers))
+
+
+# head sizes of the prompts' kernel by pairs and of the fused q, k, v product of 17 to 32 rows, in steps of each kind of
+# product, of prompts beside a few tokens (as tiles and by split keys); blocks without post norms, other activations,
+# no rotation, norm scales in 32 bits
+@pytest.mark.parametrize("heads,kv_heads,dim,form,float32_scales", [
+    (4, 2, 256, {}, False), (8, 2, 128, {}, False), (4, 2, 256, dict(block="pre_norm", activation="silu"), True),
+    (8, 2, 128, dict(block="pre_norm", activation="clamped_swish", limit=7.0, position=False), False),
+    (4, 4, 64, dict(activation="relu", position=False), True)])
+def test_layers_in_one_call_as_the_parts_make_them(monkeypatch, heads, kv_heads, dim, form, float32_scales):
+  d = design_bench.DICTS["gemma2"](dict(width=256, heads=heads, kv_heads=kv_heads, dim=dim, ff=384, vocab=512, layers=3))
+  d.update(sliding_window=100, layer_types=["sliding_attention", "full_attention", "sliding_attention"])
+  spec = _rearranged(config_from_dict(d).model_spec(), **form)
+  tensors = random_tensors(DecoderModel(spec).tensor_specs(), 3, matrix_std=0.1, scale_std=0.1, dtype=torch.bfloat16, device="cuda")
+  if float32_scales:
+    tensors = {n: t.float() if t.dim() == 1 else t for n, t in tensors.items()}
+  steps = [[9], [3, 1], [14, 5, 1], [20], [40, 30, 1], [1, 1, 28], [150, 3, 200], [1, 90, 1], [400, 1, 1]]
+  got, ran = {}, []
+  run = UniformLayers.run
+  monkeypatch.setattr(UniformLayers, "run", lambda self, *a: ran.append(run(self, *a)) or ran[-1])
+  for together in (True, False):
+    engine = Engine(types.SimpleNamespace(model_spec=lambda: spec), tensors, EngineConfig(
+        activation_dtype="bfloat16", page_size=64, batch_size=4, max_seq_len=1024, max_num_issue_tokens=512), device="cuda")
+    engine.ops.layer_runs = together
+    slots = [engine.open_request(i) for i in range(3)]
+    rng = np.random.default_rng(1)
+    rows = got[together] = []
+    for lengths in steps:
+      before = engine.ops.launches
+      logits = engine.step_raw([StepEntry(s, rng.integers(0, 512, n).tolist(), (n - 1,)) for s, n in zip(slots, lengths)])
+      rows.append((logits, engine.ops.launches - before))
+    engine.ops.check_errors()
+  assert len(ran) == len(steps) and all(b is not None for b in ran)
+  for lengths, (a, n), (b, m) in zip(steps, got[True], got[False]):
+    assert torch.isfinite(a).all() and torch.equal(a, b) and n == m, lengths
