@@ -1,12 +1,12 @@
 // Decode attention over the paged cache for single tokens and few keys (bfloat16 in, float32 arithmetic): one launch,
-// no work list, compiled once per head size (-DSB_HEAD_DIM=N): heads of 256 in groups of 2 and of 128 in groups of 4.
+// no work list, compiled once per head size (-DSB_HEAD_DIM=N; head sizes 64, 128 and 256).
 //
 //   s = q . k, s = cap tanh(s / cap) if cap > 0, keep the window's keys, o = softmax(s) . v, as attention_mma.cu
 //
 // With a few hundred keys per request the split-key kernel of attention_mma.cu is bound by what comes one after the
 // other: work items from a counter, a tile by TMA, matrix products, partial results through memory, a second launch
-// that merges them.  Here a cluster of 1 to 16 blocks owns one (request, kv head).  A warp takes tiles of 4 keys (8 of
-// heads of 128): a lane copies 16 bytes of each key row and value row for itself alone, so that nothing but
+// that merges them.  Here a cluster of 1 to 16 blocks owns one (request, kv head).  A warp takes tiles of 4 keys (8 or 16
+// of smaller heads): a lane copies 16 bytes of each key row and value row for itself alone, so that nothing but
 // its own copies has to be waited for, two tiles ahead and the first ones before the kernel waits for its
 // queries (tiles below the new token's are older than the step).  Scores are sums over lanes; weights stay in 32 bits.
 // The warps' results meet in shared memory, the blocks' through the cluster's.
@@ -34,8 +34,7 @@
 namespace {
 
 constexpr int DH = SB_HEAD_DIM;
-constexpr bool TAKES = DH == 128 || DH == 256;
-constexpr int GROUP = DH == 256 ? 2 : 4;  // query heads per kv head
+constexpr bool TAKES = DH == 64 || DH == 128 || DH == 256;
 constexpr int WARPS = 16;
 constexpr int LD = 4;      // copies per lane and tile, of keys and of values
 constexpr int STAGES = 2;  // tiles on their way per warp: 128 KB a block
@@ -82,7 +81,8 @@ struct RowsParams {
       : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
 }
 
-template <int G>  // (GROUP; a template so that it is compiled for the sizes it takes only)
+// G: query heads per kv head.
+template <int G>
 __global__ void __launch_bounds__(WARPS * 32, 1) attn_rows_kernel(const RowsParams p) {
   constexpr int LPK = DH / 8, KPI = 32 / LPK;  // lanes per key, keys per load of a warp
   constexpr int TK = LD * KPI;                 // keys per tile
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) attn_rows_kernel(const RowsPara
   const size_t v_offset = (size_t)p.num_kv_heads * page_size * DH;
   extern __shared__ __align__(16) uint4 ring[];  // [STAGES][keys, values][LD][threads]
   float (*s_o)[G][DH] = reinterpret_cast<float (*)[G][DH]>(ring);  // [WARPS], once all tiles have been read
-  static_assert(WARPS * G * DH * (int)sizeof(float) <= RING_BYTES, "the warps' results take the ring's place");
+  static_assert(WARPS * 4 * DH * (int)sizeof(float) <= RING_BYTES, "the warps' results take the ring's place");
   auto place = [&](int stage, int value, int u) { return ring + (((stage * 2 + value) * LD + u) * (WARPS * 32)) + threadIdx.x; };
   const int* table = p.block_table + (size_t)b * p.max_pages;
   // (a tile lies in one page)
@@ -158,12 +158,12 @@ __global__ void __launch_bounds__(WARPS * 32, 1) attn_rows_kernel(const RowsPara
     for (int e = 0; e < 4; ++e) o[g][e] = make_float2(0.f, 0.f);
   }
   // The sums over a key's lanes: VALUES numbers (place u * G + g: key u, head g) are halved between two halves of the
-  // lanes as long as a lane has more than one, so that a score is capped by one lane and then given to all.
-  constexpr int VALUES = LD * G;
-  static_assert(VALUES <= LPK, "a lane ends up with one score");
-  int held = 0;  // the place this lane ends up with
+  // lanes as long as a lane has more than one, so that a score is capped by one lane (two of a head of 64) and
+  // then given to all.
+  constexpr int VALUES = LD * G, HELD = VALUES > LPK ? VALUES / LPK : 1;
+  int held = 0;  // the first place this lane ends up with
 #pragma unroll
-  for (int off = LPK / 2, n = VALUES / 2; off > 0 && n > 0; off >>= 1, n >>= 1) held += lane & off ? n : 0;
+  for (int off = LPK / 2, n = VALUES / 2; off > 0 && n >= HELD && n > 0; off >>= 1, n >>= 1) held += lane & off ? n : 0;
   const float inv_cap = p.cap > 0.f ? 1.0f / p.cap : 0.f;
   for (int stage = 0; tile < tiles; tile += step, stage = stage + 1 == STAGES ? 0 : stage + 1) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 1) : "memory");
@@ -203,15 +203,19 @@ __global__ void __launch_bounds__(WARPS * 32, 1) attn_rows_kernel(const RowsPara
         s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
       }
     }
-    const int j = (tile0 + tile) * TK + held / G * KPI + sub;
-    float x = p.cap > 0.f ? p.cap * tanh_fast(s[0] * inv_cap) : s[0];
-    x = j >= lo && j < hi ? x * LOG2E : -INFINITY;
+    float x[HELD];
+#pragma unroll
+    for (int i = 0; i < HELD; ++i) {
+      const int j = (tile0 + tile) * TK + (held + i) / G * KPI + sub;
+      x[i] = p.cap > 0.f ? p.cap * tanh_fast(s[i] * inv_cap) : s[i];
+      x[i] = j >= lo && j < hi ? x[i] * LOG2E : -INFINITY;
+    }
 #pragma unroll
     for (int i = 0; i < VALUES; ++i) {
       int from = 0;
 #pragma unroll
-      for (int off = LPK / 2, n = VALUES / 2; off > 0 && n > 0; off >>= 1, n >>= 1) from |= i & n ? off : 0;
-      s[i] = __shfl_sync(0xffffffffu, x, sub * LPK + from);
+      for (int off = LPK / 2, n = VALUES / 2; off > 0 && n >= HELD && n > 0; off >>= 1, n >>= 1) from |= i & n ? off : 0;
+      s[i] = __shfl_sync(0xffffffffu, x[i % HELD], sub * LPK + from);
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -383,7 +387,7 @@ int launch(const RowsParams& p, int blocks, int cluster, cudaStream_t stream) {
 static bool cluster_size(int cluster) { return cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8 || cluster == 16; }
 
 // One token for each of `batch` requests, row b of q and out; cluster: blocks per (request, kv head), 1, 2, 4, 8 or 16.
-// Returns -9 for what it does not take (other head sizes and groups, pages of no
+// Returns -9 for what it does not take (other head sizes, groups other than 2 and 4, pages of no
 // power of two or shorter than a tile of keys, clusters that the device has no room for).
 extern "C" int SB_FN(sb_attn_rows)(const void* q, const void* cache, const int* block_table, int max_pages, const int* q_start,
                                    void* out, int batch, int num_q_heads, int num_kv_heads, int page_size, int num_pages,
@@ -392,7 +396,7 @@ extern "C" int SB_FN(sb_attn_rows)(const void* q, const void* cache, const int* 
   if (batch == 0) return 0;
   if (num_kv_heads <= 0 || num_q_heads % num_kv_heads) return -8;
   const int group = num_q_heads / num_kv_heads;
-  if (group != GROUP || page_size <= 0 || page_size < LD * 256 / DH || (page_size & (page_size - 1)) ||
+  if ((group != 2 && group != 4) || page_size <= 0 || page_size < LD * 256 / DH || (page_size & (page_size - 1)) ||
       !cluster_size(cluster) || ((uintptr_t)q & 15) || ((uintptr_t)cache & 15))
     return -9;
   int shift = 0;
@@ -401,6 +405,9 @@ extern "C" int SB_FN(sb_attn_rows)(const void* q, const void* cache, const int* 
                      num_pages, window, older_keys_settled, cap, err};
   const long long blocks = (long long)batch * num_kv_heads * cluster;
   if (blocks > 0x7fffffffLL) return -6;
-  if constexpr (TAKES) return launch<GROUP>(p, (int)blocks, cluster, stream);
+  if constexpr (TAKES) {
+    if (group == 2) return launch<2>(p, (int)blocks, cluster, stream);
+    return launch<4>(p, (int)blocks, cluster, stream);
+  }
   return -9;
 }

@@ -65,7 +65,8 @@ def attention_cluster(requests: int, kv_heads: int, group: int, dim: int, keys: 
                                  4 x 1,900 1,641 / 1,685    16 x 900  2,119 / 2,068    40 x 900 3,088 / 3,365
       Gemma 2 9B: 1 x 900 4,201 / 4,070, 8 x 900 4,634 / 4,572
       heads of 128, four to a kv head: 8 kv heads 1 x 900 487 / 468, 2 x 900 478 / 470, 3 x 900 472 / 473, 4 x 900 475 / 483
-      (4 x 300 497 / 484), 6 x 900 509 / 509, 8 x 900 545 / 558; 4 kv heads 1 x 900 594 / 602"""
+      (4 x 300 497 / 484), 6 x 900 509 / 509, 8 x 900 545 / 558; 4 kv heads 1 x 900 594 / 602
+  Other heads and groups that the kernel is compiled for have no measured step: they stay with the split keys."""
   pairs = requests * kv_heads
   cluster = max((c for c in (1, 2, 4, 8, 16) if pairs * c <= (64 if c >= 8 else 128)), default=0) or int(pairs <= SMS)
   if not cluster or keys > (256 * cluster if cluster >= 4 else 1024):

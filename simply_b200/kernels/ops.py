@@ -499,7 +499,7 @@ class CudaOps:
                                  c_int, c_float, c_int, c_void, c_int, c_void, c_void]
         prefill_pair.restype = c_int
       rows = None
-      if head_dim in (128, 256) and value_dim == head_dim:
+      if head_dim in (64, 128, 256) and value_dim == head_dim:
         rows = getattr(lib, f"sb_attn_rows_{suffix}")
         rows.argtypes = [c_void, c_void, c_void, c_int, c_void, c_void, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
                          c_int, c_int, c_void, c_void]
