@@ -76,11 +76,12 @@ def attention_cluster(requests: int, kv_heads: int, group: int, dim: int, keys: 
   return cluster if dim == 128 and group == 4 and 8 <= pairs <= 16 else 0
 
 
-def few_rows_join_tiles(keys: Sequence[int], prompt_keys: Sequence[int], kv_heads: int, rows: int, key_bytes: int) -> bool:
+def few_rows_join_tiles(keys: Sequence[int], kv_heads: int, prompt_keys: Sequence[int] = (100,), rows: int = 0,
+                        key_bytes: int = 1024) -> bool:
   """Whether the requests of a step that bring only a few tokens beside prompts (`keys`: how many each sees) are tiles of
   the prompts' attention kernel too (csrc/attention_tc_pair.cu), in place of a split-key launch and its merge behind
-  it.  `prompt_keys`: the keys of each of the prompts' tiles; `rows`: the step's tokens times query heads; `key_bytes`: of a
-  key and its value.
+  it.  `prompt_keys`: the keys of each of the prompts' tiles (one short prompt where they are not given); `rows`: the step's
+  tokens times query heads; `key_bytes`: of a key and its value (heads of 256).
 
   A tile is walked from end to end by one of 74 pairs of blocks: 9 us and 14.5 us per 1,000 keys (19 with a prompt's
   full rows), for heads of 128 and 256 alike.  So a lone request of many keys is the longest walk of the step unless a

@@ -702,7 +702,7 @@ class CudaOps:
     pre = tiles(np.nonzero(~small)[0])
     if force_rows == 256 and self.few_rows_in_tiles and pre and small.any():
       few = tiles(np.nonzero(small)[0])
-      if few_rows_join_tiles([t[0] for t in few], [t[0] for t in pre], num_kv_heads, int(cu_q[-1]) * num_kv_heads * group,
+      if few_rows_join_tiles([t[0] for t in few], num_kv_heads, [t[0] for t in pre], int(cu_q[-1]) * num_kv_heads * group,
                              4 * head_dim):
         pre += few
         small[:] = False

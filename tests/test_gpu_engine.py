@@ -242,6 +242,9 @@ def test_engine_refuses_without_cuda_kernels(monkeypatch):
 @pytest.mark.parametrize("width,hidden,kv_heads", [(256, 384, 2), (256, 388, 1), (260, 384, 2)])
 @pytest.mark.parametrize("steps", [[[9]], [[16, 1]], [[20, 5], [1, 30]], [[60, 41, 2], [1, 1, 9]], [[150, 3], [1, 140]]])
 def test_layers_in_one_call_give_the_same_bits(monkeypatch, width, hidden, kv_heads, steps):
+  from simply_b200 import design_bench
+  from simply_b200.config import config_from_dict
+  from simply_b200.kernels.layer_run import UniformLayers
   d = design_bench.DICTS["gemma2"](dict(width=width, heads=4, kv_heads=kv_heads, dim=64, ff=hidden, vocab=512, layers=3))
   d.update(sliding_window=48, layer_types=["sliding_attention", "full_attention", "sliding_attention"])
   ran = []

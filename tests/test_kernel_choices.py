@@ -141,6 +141,14 @@ def test_decode_attention_in_one_launch_is_refused_where_no_cluster_fits():
   assert done.stdout.split("\n")[-2] == str([-9] * 5), done.stdout + done.stderr
 
 
+# requests of one token, their keys: us of a step with them on split keys and as tiles beside a prompt
+@pytest.mark.parametrize("requests,keys,times", [
+    (8, 200, (2673, 2295)), (8, 600, (3579, 3141)), (16, 200, (2872, 2464)), (16, 600, (3898, 3541)), (39, 100, (3013, 3034)),
+    (39, 300, (3213, 3305)), (39, 600, (3492, 3590)), (1, 3, (14001, 13230))])
+def test_few_rows_are_tiles_where_that_is_faster(requests, keys, times):
+  assert few_rows_join_tiles([keys] * requests, 4) == (times[1] < times[0])
+
+
 # heads, kv heads, head size, the prompt, requests of one token and their keys: us of a layer's attention by split keys and
 # as tiles
 @pytest.mark.parametrize("heads,kv_heads,dim,prompt,requests,keys,times", [
@@ -155,10 +163,10 @@ def test_decode_attention_in_one_launch_is_refused_where_no_cluster_fits():
     (32, 8, 128, 400, 32, 600, (62.5, 82.1)), (32, 8, 128, 1500, 1, 4000, (126.0, 71.7)), (32, 8, 128, 4000, 32, 600, (416.8, 317.4)),
     (16, 4, 128, 60, 1, 1000, (25.6, 28.7)), (16, 4, 128, 60, 16, 1000, (31.7, 30.7)), (16, 4, 128, 400, 1, 8000, (41.7, 120.8)),
     (16, 4, 128, 1500, 1, 4000, (76.8, 70.5)), (16, 4, 128, 4000, 1, 8000, (216.1, 140.3))])
-def test_few_rows_are_tiles_where_that_is_faster(heads, kv_heads, dim, prompt, requests, keys, times):
+def test_few_rows_are_tiles_where_a_layer_is_faster_for_it(heads, kv_heads, dim, prompt, requests, keys, times):
   tile = 256 // (heads // kv_heads)
   prompts = [min(i + tile, prompt) for i in range(0, prompt, tile)]
-  joined = few_rows_join_tiles([keys + 1] * requests, prompts, kv_heads, (prompt + requests) * heads, 4 * dim)
+  joined = few_rows_join_tiles([keys + 1] * requests, kv_heads, prompts, (prompt + requests) * heads, 4 * dim)
   assert times[joined] <= 1.04 * min(times)
 
 
