@@ -666,7 +666,7 @@ class CudaOps:
     """Work lists of the two tensor-core kernels for this step, per kind of layer (`_plan_key`) and kernel for its
     prompts: `force_rows` 256 the tcgen05 kernel by pairs, 128 the one by single blocks, 0 the mma.sync kernel.  Their
     tiles differ, and with them which requests the split-key kernel is left with: layers share a list only if
-    their prompts go to the same kernel.
+    their prompts go to the same kernel, or if the step has none.
 
     Sequences with at most 16 query rows per kv head (one or a few new tokens) go to the
     split-key kernel: their keys are cut into chunks at multiples of `chunk` of the
@@ -674,9 +674,11 @@ class CudaOps:
     64 // group or 128 // group tokens for the prefill kernel, heaviest tile first.
     """
     key = self._plan_key(window, group, num_kv_heads, head_dim, key_chunk, value_dim, keep_first)
-    plan = ctx.memo.get(key)  # (a decode graph brings its static list)
+    plan = ctx.memo.get(key) if not tag else None  # (a decode graph brings its static list)
     if plan is not None:
       return plan
+    if ctx.max_q_len * group <= 16 and not all_tiles:
+      force_rows = 0  # (no tiles: one list for every kind)
     key += ("prompts", force_rows) + tag
     plan = ctx.memo.get(key)
     if plan is not None:

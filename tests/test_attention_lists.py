@@ -87,3 +87,20 @@ def test_every_row_is_computed_once_whatever_layers_share_a_step(seqs, window):
       ops.paged_attention(q, storage, torch.zeros(len(seqs), 16, dtype=torch.int32), ctx, num_heads=HEADS, num_kv_heads=KV_HEADS,
                           head_dim=DIM, logit_softcap=cap, window=window, **options)
       assert (launches.covered == 1).all(), (first, second, name)
+
+
+def test_steps_of_few_tokens_alone_have_one_list():
+  """Without prompts there are no tiles, and every kind of layer reads the same split keys: they are listed once."""
+  launches = Launches([1, 1, 2])
+  ops = host_table(launches)
+  q, storage = torch.zeros(4, HEADS, DIM, dtype=torch.bfloat16), torch.zeros(16, 2, KV_HEADS, PAGE, DIM, dtype=torch.bfloat16)
+  ints = torch.zeros(4, dtype=torch.int32)
+  ctx = types.SimpleNamespace(
+      host=dict(cu_q=launches.cu, q_start=np.array([300, 0, 700])), memo={}, page_size=PAGE, num_seqs=3, num_tokens=4, max_q_len=2,
+      max_kv_len=702, cu_q=ints, q_start=ints, token_seq=ints, positions=ints)
+  for name, (options, cap) in KINDS.items():
+    launches.clear()
+    ops.paged_attention(q, storage, torch.zeros(3, 16, dtype=torch.int32), ctx, num_heads=HEADS, num_kv_heads=KV_HEADS,
+                        head_dim=DIM, logit_softcap=cap, window=None, **options)
+    assert (launches.covered == 1).all(), name
+  assert len(ctx.memo) == 1
