@@ -1120,7 +1120,6 @@ class CudaOps:
     value_dim = head_dim if value_dim is None else value_dim
     out = self._new(t, num_heads * value_dim, dtype=q.dtype)
     group = num_heads // num_kv_heads
-    together = tokens_per_attention_block(t, ctx.num_seqs, num_heads)  # (of the general kernel)
     if (values_in_keys or key_chunk is not None) and (logit_softcap or pooled is not None):
       raise KernelError("latent rows and chunks of keys go with neither a score cap nor pooled blocks")
     if sink is not None and pooled is not None:
@@ -1150,7 +1149,8 @@ class CudaOps:
                    block_table.shape[1], _ptr(ctx.token_seq), _ptr(ctx.positions), _ptr(out), t, num_heads,
                    num_kv_heads, head_dim, value_dim, ctx.page_size, storage.shape[0], float(logit_softcap),
                    int(window or 0), *pool_args, int(values_in_keys), _ptr(sink), _ptr(distance_bias), linear_bias,
-                   int(key_chunk or 0), keep_first, _ptr(ctx.cu_q), ctx.num_seqs, together, _ptr(self.err))
+                   int(key_chunk or 0), keep_first, _ptr(ctx.cu_q), ctx.num_seqs,
+                   tokens_per_attention_block(t, ctx.num_seqs, num_heads), _ptr(self.err))
 
       # bfloat16 with key size = value size: the tensor-core tile kernel (mma.sync tiles of 64 rows,
       # the block entries in tiles of their own ahead of the tokens) for prompt portions and single
@@ -1271,7 +1271,8 @@ class CudaOps:
     self._call("sb_paged_attention_generic", _ptr(q), _code(q), _ptr(storage), _ptr(block_table),
                block_table.shape[1], _ptr(ctx.token_seq), _ptr(ctx.positions), _ptr(out), t, num_heads,
                num_kv_heads, head_dim, ctx.page_size, storage.shape[0], float(logit_softcap),
-               int(window or 0), _ptr(ctx.cu_q), ctx.num_seqs, together, _ptr(self.err))
+               int(window or 0), _ptr(ctx.cu_q), ctx.num_seqs, tokens_per_attention_block(t, ctx.num_seqs, num_heads),
+               _ptr(self.err))
     return out
 
   # ---- attention with normed queries and keys ---------------------------------

@@ -104,3 +104,10 @@ def test_steps_of_few_tokens_alone_have_one_list():
                         head_dim=DIM, logit_softcap=cap, window=None, **options)
     assert (launches.covered == 1).all(), name
   assert len(ctx.memo) == 1
+
+
+def test_only_the_general_kernel_asks_how_many_tokens_share_a_block(monkeypatch):
+  def refused(*a):
+    raise AssertionError("asked for a tensor-core kernel")
+  monkeypatch.setattr("simply_b200.kernels.ops.tokens_per_attention_block", refused)
+  test_steps_of_few_tokens_alone_have_one_list()
