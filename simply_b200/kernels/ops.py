@@ -691,22 +691,19 @@ class CudaOps:
     tokens_per_tile = rows_per_tile // group
     num_seqs = len(q_len)
 
-    def tiles(seqs: np.ndarray) -> list:
-      got = []
-      for b in seqs:
-        for i0 in range(0, int(q_len[b]), tokens_per_tile):
-          last = int(q_start[b]) + min(i0 + tokens_per_tile, int(q_len[b]))
-          at = int(q_start[b]) + i0
-          first = max(at - window + 1, 0) if window else at // key_chunk * key_chunk if key_chunk else 0
-          got.append((last - first + min(keep_first, first), int(b), i0))
-      return got
-
-    pre = tiles(np.nonzero(~small)[0])
+    low = self.lowest_keys(q_start, window, key_chunk)
+    pre = []
+    for b in np.nonzero(~small)[0]:
+      for i0 in range(0, int(q_len[b]), tokens_per_tile):
+        last = int(q_start[b]) + min(i0 + tokens_per_tile, int(q_len[b]))
+        at = int(q_start[b]) + i0
+        first = max(at - window + 1, 0) if window else at // key_chunk * key_chunk if key_chunk else 0
+        pre.append((last - first + min(keep_first, first), int(b), i0))
     if force_rows == 256 and self.few_rows_in_tiles and pre and small.any():
-      few = tiles(np.nonzero(small)[0])
-      if few_rows_join_tiles([t[0] for t in few], num_kv_heads, [t[0] for t in pre], int(cu_q[-1]) * num_kv_heads * group,
-                             4 * head_dim):
-        pre += few
+      few = np.nonzero(small)[0]
+      keys = (q_start + q_len - low)[few].tolist()  # (a request of a few tokens is one tile)
+      if few_rows_join_tiles(keys, num_kv_heads, [t[0] for t in pre], int(cu_q[-1]) * num_kv_heads * group, 4 * head_dim):
+        pre += [(k, b, 0) for k, b in zip(keys, few.tolist())]
         small[:] = False
     pre.sort(key=lambda x: -x[0])
     if force_rows in (128, 256):
@@ -719,7 +716,7 @@ class CudaOps:
     else:
       prefill_items = np.array([(b, i0) for _, b, i0 in pre], dtype=np.int32).reshape(-1, 2)
     kv_hi = q_start + q_len
-    kv_lo = self.lowest_keys(q_start, window, key_chunk) // 64 * 64
+    kv_lo = low // 64 * 64
     dec = np.nonzero(small)[0]
     chunk = 64
     if len(dec):
