@@ -12,6 +12,8 @@
 // 8 x 16 or 16 x 8 (one output per thread) fed by a deep ring of asynchronous copies for up to 16 rows, where
 // the weights only stream by.  sb_gemm_f32_tile has the lines between them; sb_gemm_f32_groups says whether a
 // tile's quarters of k are four groups of a block's threads.
+#include <type_traits>
+
 #include "common.cuh"
 
 // Two FMAs in one instruction, each rounded as fmaf rounds.
@@ -52,13 +54,17 @@ __device__ __forceinline__ float4 row_quad(const float* __restrict__ p, bool in,
 // What bounds it: a warp's reads of shared memory deliver 128 bytes a cycle and SM, so TM + TN cycles per
 // k beside TM TN / 4 cycles of FMAs: 16 x 8 outputs per thread keep the FMA pipes the longer of the two,
 // 8 x 8 are even, and 8 x 4 are half as long again as their FMAs.  64 x 64 of 8 x 4 all the same, whose blocks of
-// 128 threads stand four to an SM: with 8 x 8 per thread 256 x 16,384 x 2,048 took 425 us (G = 4: 467) in place of 358.
+// 128 threads stand four to an SM: with 8 x 8 per thread 256 x 16,384 x 2,048 took 425 us (GROUPS 4: 467) in place of 351.
+// One group walks all of k as one pipeline: a pipeline per quarter waited for its first tile four times (6,000 x 16,384 x
+// 64 329 us in place of 308).  Four blocks to an SM only if the compiler is held to 128 registers: 3 blocks of 134 335 us.
+// The sums so far pass through shared memory, at 256 bytes per thread and quarter: rows of a few tiles pay for it
+// (6,000 x 2,048 x 100 81 us, as one chain 75; x 256 142 and 138; x 2,048 and longer nothing).
 // ---------------------------------------------------------------------------
 // A quarter of k, in whole tiles of 32.
 __host__ __device__ __forceinline__ int f32_quarter(int K) { return (K + 127) / 128 * 32; }
 
 template <int BM, int BN, int BK, int TM, int TN, int GROUPS>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN) * GROUPS)
+__global__ void __launch_bounds__((BM / TM) * (BN / TN) * GROUPS, BM == 64 && GROUPS == 1 ? 4 : BM == 128 ? 1 : 0)
 gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out, int M, int N,
                      int K, float cap, int vec) {
   constexpr int THREADS = (BM / TM) * (BN / TN), QUADS = BK / 4;  // (threads of a group)
@@ -87,8 +93,7 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, f
   auto turn = [](int q) { return (q % 4) * 8 + (q / 4) * 4; };
   constexpr int STEP = THREADS / QUADS;  // rows between a thread's pieces
   float4 xq[XQ], wq[WQ];
-  int k_end = 0;  // of the quarter that is walked (at most K)
-  auto fetch = [&](int k0) {
+  auto fetch = [&](int k0, int k_end) {
 #pragma unroll
     for (int i = 0; i < XQ; ++i) {
       const int r = m0 + row + i * STEP;
@@ -114,70 +119,75 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, f
   };
   float2 acc[TM / 2][TN];
   float* sums = tile_smem + TILE_FLOATS + tid;  // GROUPS 1: this thread's sums so far, THREADS apart
-  const int quarter = f32_quarter(K), parts = GROUPS == 1 ? (K + quarter - 1) / max(quarter, 1) : 4;  // (empty quarters add nothing)
-#pragma unroll 1
-  for (int part = GROUPS == 1 ? 0 : group; part < max(parts, 1); part += GROUPS) {
-    const int k_start = min(part * quarter, K);
-    k_end = min(k_start + quarter, K);
+  const int quarter = f32_quarter(K);
+  const int k_start = GROUPS == 1 ? 0 : min(group * quarter, K), k_end = GROUPS == 1 ? K : min(k_start + quarter, K);
+#pragma unroll
+  for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  if (k_start < k_end) {
+    fetch(k_start, k_end);
+    put(0);
+  }
+  meet();
+  int next_quarter = quarter;  // where the next chain begins
+  auto add_sums = [&]() {
 #pragma unroll
     for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
-    if (k_start < k_end) {
-      fetch(k_start);
-      put(0);
-    }
-    meet();
-    for (int k0 = k_start, buf = 0; k0 < k_end; k0 += BK, buf ^= 1) {
-      const bool more = k0 + BK < k_end;
-      if (more) fetch(k0 + BK);
-      float2 a[2][TM / 2];
-      float b[2][TN];
-      auto read = [&](int s, int k) {
-        const int at = turn(k / 4);
-#pragma unroll
-        for (int i = 0; i < TM; i += 4) {
-          const float4 v = *reinterpret_cast<const float4*>(&xs[buf][k][(mt + i) ^ at]);
-          a[s][i / 2] = make_float2(v.x, v.y);
-          a[s][i / 2 + 1] = make_float2(v.z, v.w);
-        }
-#pragma unroll
-        for (int j = 0; j < TN; j += 4) {
-          const float4 v = *reinterpret_cast<const float4*>(&ws[buf][k][(nt + j * 8) ^ at]);
-          b[s][j] = v.x; b[s][j + 1] = v.y; b[s][j + 2] = v.z; b[s][j + 3] = v.w;
-        }
-      };
-      read(0, 0);
-#pragma unroll
-      for (int k = 0; k < BK; ++k) {  // (values beyond the end are zeros on both sides: the chain keeps its value)
-        if (k + 1 < BK) read((k + 1) & 1, k + 1);
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          const float2 bb = make_float2(b[k & 1][j], b[k & 1][j]);
-#pragma unroll
-          for (int i = 0; i < TM / 2; ++i) fma_pair(acc[i][j], a[k & 1][i], bb);
-        }
+      for (int j = 0; j < TN; ++j) {
+        const float* at = sums + (i * TN + j) * 2 * THREADS;
+        acc[i][j].x = at[0] + acc[i][j].x;
+        acc[i][j].y = at[THREADS] + acc[i][j].y;
       }
-      if (more) put(buf ^ 1);
-      meet();
+  };
+  for (int k0 = k_start, buf = 0; k0 < k_end; k0 += BK, buf ^= 1) {
+    const bool more = k0 + BK < k_end;
+    if (more) fetch(k0 + BK, k_end);
+    float2 a[2][TM / 2];
+    float b[2][TN];
+    auto read = [&](int s, int k) {
+      const int at = turn(k / 4);
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&xs[buf][k][(mt + i) ^ at]);
+        a[s][i / 2] = make_float2(v.x, v.y);
+        a[s][i / 2 + 1] = make_float2(v.z, v.w);
+      }
+#pragma unroll
+      for (int j = 0; j < TN; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(&ws[buf][k][(nt + j * 8) ^ at]);
+        b[s][j] = v.x; b[s][j + 1] = v.y; b[s][j + 2] = v.z; b[s][j + 3] = v.w;
+      }
+    };
+    read(0, 0);
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {  // (values beyond the end are zeros on both sides: the chain keeps its value)
+      if (k + 1 < BK) read((k + 1) & 1, k + 1);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        const float2 bb = make_float2(b[k & 1][j], b[k & 1][j]);
+#pragma unroll
+        for (int i = 0; i < TM / 2; ++i) fma_pair(acc[i][j], a[k & 1][i], bb);
+      }
     }
-    if (GROUPS == 1) {
+    if (GROUPS == 1 && more && k0 + BK == next_quarter) {  // (a chain has ended; the next tiles are on their way)
+      if (next_quarter > quarter) add_sums();
 #pragma unroll
       for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
           float* at = sums + (i * TN + j) * 2 * THREADS;
-          if (part > 0) {
-            acc[i][j].x = at[0] + acc[i][j].x;
-            acc[i][j].y = at[THREADS] + acc[i][j].y;
-          }
-          if (part + 1 < parts) {
-            at[0] = acc[i][j].x;
-            at[THREADS] = acc[i][j].y;
-          }
+          at[0] = acc[i][j].x;
+          at[THREADS] = acc[i][j].y;
+          acc[i][j] = make_float2(0.f, 0.f);
         }
+      next_quarter += quarter;
     }
+    if (more) put(buf ^ 1);
+    meet();
   }
+  if (GROUPS == 1 && next_quarter > quarter) add_sums();
   if (GROUPS == 1) {
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
@@ -215,10 +225,13 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, f
 // ---------------------------------------------------------------------------
 // Up to 16 rows: one output per thread, 128 per block (ROWS x 128 / ROWS).  The weights' rows stream
 // through a ring of asynchronous 16-byte copies (rows of 16-byte multiples only), several blocks per
-// SM; a thread walks the four quarters' chains side by side (one chain's FMA waits 4 cycles for the one before).
+// SM; a thread has the vectors of the next 16 k in registers while it multiplies these.  The four quarters' chains one
+// after the other: side by side a stage held 32 k of each, and took longer although the FMAs wait less for one another
+// (us, side by side and so: 1 x 16,384 x 2,048 44.8 and 42.2, x 2,048 x 8,192 49.2 and 45.3; 8 x 16,384 x 2,048 78.6 and
+// 76; 9 117.8 and 121; 16 138 and 127.5, x 2,048 x 8,192 102.7 and 102.3).
 // ---------------------------------------------------------------------------
 #define F32_FEW 16        // most rows
-#define F32_FEW_K 128     // k per stage: 32 of each quarter
+#define F32_FEW_K 128     // k per stage
 #define F32_FEW_STAGES 5
 #define F32_FEW_LD (F32_FEW_K + 4)  // a row's start moves on by 4 banks
 
@@ -229,14 +242,13 @@ gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
   constexpr int COLS = 128 / ROWS, STAGE = (COLS + ROWS) * F32_FEW_LD, PIECES = F32_FEW_K / 4;
   extern __shared__ __align__(16) float few_smem[];  // stages of (weights [COLS][LD], x [ROWS][LD])
   const int n0 = blockIdx.x * COLS;
-  const int quarter = f32_quarter(K), steps = quarter / 32;
+  const int steps = (K + F32_FEW_K - 1) / F32_FEW_K, quarter = f32_quarter(K);
   // A warp copies a row's 512 bytes at a time.  (Beyond the matrix: 0 bytes read, zeros written.)
   const int piece = (threadIdx.x % PIECES) * 4, first = threadIdx.x / PIECES;
-  const int from_k = piece / 32 * quarter + piece % 32, end_k = min(piece / 32 * quarter + quarter, K);
   auto copy = [&](const float* from, int rows, int count, int step, float* to) {
-    const int k = step * 32 + from_k;
+    const int k = step * F32_FEW_K + piece;
     for (int r = first; r < count; r += 128 / PIECES) {
-      const bool in = r < rows && k < end_k;
+      const bool in = r < rows && k < K;
       const float* src = in ? from + (size_t)r * K + k : from;
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
                        (unsigned)__cvta_generic_to_shared(to + r * F32_FEW_LD + piece)), "l"(src), "r"(in ? 16 : 0));
@@ -253,7 +265,13 @@ gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
     asm volatile("cp.async.commit_group;\n");
   }
   const int m = threadIdx.x / COLS, n = threadIdx.x % COLS;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  float acc = 0.f, sum = 0.f;  // the chain that is walked, the ones that have ended
+  int left = quarter;          // of this chain's k
+  auto ended = [&]() {
+    sum += acc;
+    acc = 0.f;
+    left = quarter;
+  };
   for (int s = 0; s < steps; ++s) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(F32_FEW_STAGES - 2));
     __syncthreads();  // the stage has landed for all; the one read a turn ago is free
@@ -264,34 +282,45 @@ gemm_f32_few_kernel(const float* __restrict__ x, const float* __restrict__ w, fl
       copy(x, M, ROWS, next, to + COLS * F32_FEW_LD);
     }
     asm volatile("cp.async.commit_group;\n");
+    if (m >= M) continue;
     const float* wr = few_smem + (s % F32_FEW_STAGES) * STAGE + n * F32_FEW_LD;
     const float* xr = few_smem + (s % F32_FEW_STAGES) * STAGE + (COLS + m) * F32_FEW_LD;
-    if (m < M) {
+    auto walk = [&](auto count, int k0) {
+      constexpr int COUNT = decltype(count)::value;
       float4 a[2][4], b[2][4];
       auto read = [&](int at, int k) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          a[at][q] = *reinterpret_cast<const float4*>(xr + 32 * q + k);
-          b[at][q] = *reinterpret_cast<const float4*>(wr + 32 * q + k);
+          a[at][q] = *reinterpret_cast<const float4*>(xr + k + 4 * q);
+          b[at][q] = *reinterpret_cast<const float4*>(wr + k + 4 * q);
         }
       };
-      read(0, 0);
+      read(0, k0);
 #pragma unroll
-      for (int k = 0; k < 32; k += 4) {
-        const int at = (k / 4) & 1;
-        if (k + 4 < 32) read(at ^ 1, k + 4);
+      for (int k = 0; k < COUNT; k += 16) {
+        const int at = (k / 16) & 1;
+        if (k + 16 < COUNT) read(at ^ 1, k0 + k + 16);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q] = fmaf(a[at][q].x, b[at][q].x, acc[q]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q] = fmaf(a[at][q].y, b[at][q].y, acc[q]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q] = fmaf(a[at][q].z, b[at][q].z, acc[q]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q] = fmaf(a[at][q].w, b[at][q].w, acc[q]);
+        for (int q = 0; q < 4; ++q) {
+          acc = fmaf(a[at][q].x, b[at][q].x, acc);
+          acc = fmaf(a[at][q].y, b[at][q].y, acc);
+          acc = fmaf(a[at][q].z, b[at][q].z, acc);
+          acc = fmaf(a[at][q].w, b[at][q].w, acc);
+        }
+      }
+      left -= COUNT;
+    };
+    if (left >= F32_FEW_K) {
+      walk(std::integral_constant<int, F32_FEW_K>{}, 0);
+      if (left == 0) ended();
+    } else {  // a chain ends inside the stage (quarters are whole times 32)
+      for (int k = 0; k < F32_FEW_K; k += 32) {
+        walk(std::integral_constant<int, 32>{}, k);
+        if (left == 0) ended();
       }
     }
   }
-  if (m < M && n0 + n < N) out[(size_t)m * N + n0 + n] = capped(((acc[0] + acc[1]) + acc[2]) + acc[3], cap);
+  if (m < M && n0 + n < N) out[(size_t)m * N + n0 + n] = capped(sum + acc, cap);
 }
 
 template <int ROWS>
@@ -323,9 +352,9 @@ static int launch_f32_tile(const float* x, const float* w, float* out, int M, in
 
 // Rows of the tile that a product takes; `vec`: rows of whole 16-byte pieces that start on their boundaries.
 // A block of 128 x 128 fills an SM and its tile is long to set up and to store, so it needs many rounds of
-// tiles and long rows (us, 128 x 128 against 64 x 64): 256 x 16,384 x 2,048 (256 tiles) 383 and 352; 4,000 x
-// 3,100 x 2,048 (800) 1,090 and 1,031; 1,500 x 9,000 x 2,048 (852) 1,096 and 1,121, x 1,024 571 and 570, x 256
-// 181 and 151; 2,048 x 16,384 x 2,048 (2,048) 2,505 and 2,697, x 512 705 and 695; 1,500 x 3,100 x 31 26.4 and 12.1.
+// tiles and long rows (us, 128 x 128 against 64 x 64): 256 x 16,384 x 2,048 (256 tiles) 376 and 351; 4,000 x
+// 3,100 x 2,048 (800) 1,075 and 1,024; 1,500 x 9,000 x 2,048 (852) 1,079 and 1,116, x 1,024 569 and 569, x 256
+// 188 and 156; 2,048 x 16,384 x 2,048 (2,048) 2,467 and 2,678, x 512 716 and 702; 1,500 x 3,100 x 31 29.2 and 12.5.
 extern "C" int sb_gemm_f32_tile(int M, int N, int K, int vec) {
   if (M <= F32_FEW && vec && K > 0) return M <= 8 ? 8 : 16;
   auto tiles = [&](int side) { return (long long)((N + side - 1) / side) * ((M + side - 1) / side); };
@@ -334,14 +363,21 @@ extern "C" int sb_gemm_f32_tile(int M, int N, int K, int vec) {
 }
 
 // Groups of threads a tile of 64 or 32 has for the quarters of k.  Four where the tiles alone leave SMs with too few
-// warps: an SM holds one block of 4 x 128 threads, or four of 128 (us, 1 group against 4, tiles of 64: 256 x 2,048 x
-// 2,048, 128 tiles, 80 and 62, x 8,192 291 and 215; 256 x 3,072 x 2,048, 192, 117 and 113; 44 x 16,384 x 2,048, 256, 117
-// and 113; 600 x 2,048 x 8,192, 320, 631 and 602; 44 x 32,768 x 2,048, 512, 211 and 215; 256 x 16,384 x 2,048, 1,024, 358
-// and 377; 300 x 9,000 x 32 15.2 and 20.5; tiles of 32: 44 x 2,048 x 2,048 70 and 31, x 8,192 253 and 98; 300 x 500 x
-// 1,024 39 and 27; 40 x 200 x 63 10 and 8; 300 x 9,000 x 32 17 and 20).
+// warps and the quarters are long enough to share: an SM holds one block of 4 x 128 threads, or four of 128.  us, 1 group
+// against 4, tiles of 64:
+//   to one per SM   256 x 2,048 x 64 (128) 5.4 and 5.4, x 100 7.9 and 7.2, x 256 12.5 and 10.7, x 2,048 72 and 56, x 8,192 275 and 207
+//   to two          44 x 16,384 x 512 (256) 31.2 and 32.0, x 2,048 110 and 107; 256 x 3,000 x 515 (188) 35.3 and 37.1;
+//                   256 x 3,072 x 2,048 (192) 112 and 108; 600 x 1,600 x 1,024 (250) 58.6 and 57.9
+//   beyond          600 x 2,048 x 100 (320) 16.5 and 16.9, x 256 27.6 and 26.8, x 512 50 and 46, x 2,048 185 and 158, x 8,192
+//                   726 and 593; 600 x 3,072 x 2,048 (480) 209 and 208; 44 x 32,768 x 2,048 (512) 203 and 208;
+//                   256 x 16,384 x 2,048 (1,024) 351 and 369
+// and of 32: 44 x 2,048 x 2,048 56 and 26, x 8,192 230 and 96; 300 x 500 x 1,024 31 and 22; 20 x 2,048 x 64 4.5 and 3.8, x 32
+// 3.6 and 3.6.
 extern "C" int sb_gemm_f32_groups(int M, int N, int K, int tile) {
   const long long tiles = (long long)((N + 63) / 64) * ((M + 63) / 64);
-  return tile <= 64 && K > 32 && (tile == 32 || tiles < 400) ? 4 : 1;
+  if (tile == 32) return K > 32 ? 4 : 1;
+  if (tile != 64) return 1;
+  return (tiles <= 148 ? K > 64 : tiles < 400 && K >= (tiles <= 296 ? 1024 : 256)) ? 4 : 1;
 }
 
 // `tile` and `groups`: 0 for the ones that the sizes choose (others are for tests).

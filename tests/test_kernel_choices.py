@@ -64,6 +64,31 @@ def test_tiles_of_the_float32_product(lib, m, n, k, times):
   assert times[(128, 64, 32).index(got)] <= 1.05 * min(times)
 
 
+# the same with the groups of threads that the tiles now have
+@pytest.mark.parametrize("m,n,k,times", [
+    (1500, 3100, 31, (29.2, 12.5, 18.1)), (300, 9000, 32, (21.2, 8.4, 11.8)), (300, 9000, 4096, (726, 504, 713)),
+    (256, 16384, 2048, (376, 351, 508)), (44, 32768, 2048, (374, 203, 253)), (256, 2048, 8192, (809, 207, 303)),
+    (44, 2048, 8192, (803, 202, 96)), (4000, 3100, 2048, (1075, 1024, 1471)), (1500, 9000, 2048, (1079, 1116, 1611)),
+    (1500, 9000, 1024, (569, 569, 820)), (1500, 9000, 256, (188, 156, 225)), (2048, 16384, 2048, (2467, 2678, 3971)),
+    (2048, 16384, 512, (716, 701, 1035)), (6000, 16384, 64, (536, 308, 571)), (600, 1600, 1024, (115, 57.9, 68.1)),
+    (300, 500, 1024, (115, 30.2, 21.9))])
+def test_tiles_of_the_float32_product_with_their_groups(lib, m, n, k, times):
+  got = lib.sb_gemm_f32_tile(m, n, k, int(k % 4 == 0))
+  assert times[(128, 64, 32).index(got)] <= 1.05 * min(times)
+
+
+# rows, columns, k, tile: us with one and four groups of threads per tile
+@pytest.mark.parametrize("m,n,k,tile,times", [
+    (256, 2048, 64, 64, (5.4, 5.4)), (256, 2048, 100, 64, (7.9, 7.2)), (256, 2048, 256, 64, (12.5, 10.7)), (256, 2048, 2048, 64, (72, 56)),
+    (44, 16384, 512, 64, (31.2, 32.0)), (44, 16384, 2048, 64, (110, 107)), (256, 3000, 515, 64, (35.3, 37.1)), (256, 3072, 2048, 64, (112, 108)),
+    (600, 1600, 1024, 64, (58.6, 57.9)), (600, 2048, 64, 64, (9.6, 11.5)), (600, 2048, 100, 64, (16.5, 16.9)), (600, 2048, 256, 64, (27.6, 26.8)), (600, 2048, 512, 64, (50, 46)),
+    (600, 2048, 8192, 64, (726, 593)), (600, 3072, 2048, 64, (209, 208)), (44, 32768, 2048, 64, (203, 208)), (256, 16384, 2048, 64, (351, 369)),
+    (6000, 16384, 64, 64, (308, 525)), (44, 2048, 2048, 32, (56, 26)), (300, 500, 1024, 32, (31, 22)), (20, 2048, 64, 32, (4.5, 3.8)),
+    (20, 2048, 32, 32, (3.6, 3.6))])
+def test_groups_of_the_float32_product(lib, m, n, k, tile, times):
+  assert times[(1, 4).index(lib.sb_gemm_f32_groups(m, n, k, tile))] <= 1.01 * min(times)
+
+
 def _beside(prompt, singles):
   return [prompt] + [1] * singles
 
