@@ -14,9 +14,11 @@ from typing import Any
 import numpy as np
 import torch
 
+from simply_b200.kernels.ops import CudaOps
 from simply_b200.parts.attention import PagedAttention
 from simply_b200.parts.block import PreNormBlock, SandwichNormBlock
 from simply_b200.parts.feedforward import GatedFeedForward
+from simply_b200.parts.linear import Linear
 from simply_b200.parts.norm import RMSNorm
 
 _P, _I, _F, _L = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_longlong
@@ -46,9 +48,13 @@ LAYER_WORDS = 16  # numbers of 64 bits per layer
 # 3,300 in all 13,982 and 14,025; 9B, 300 tokens 10,953 and 10,941, 3,001 50,544 and 50,746).
 MOST_OPERATIONS = 1e11
 
-# What the one call stands for: a kernel table on which one of these has been replaced goes part by part.
+# What the one call stands for: where one of these has been replaced, on the kernel table, its class, a part or a part's
+# class (a tracer's or a test's), the layers go part by part.
 STANDS_FOR = frozenset(("residual_norm", "project_rotate_store", "rope_and_cache_write", "paged_attention", "linear",
                         "gated_linear", "gated_activation", "_call"))
+OWN_CALLS = [(CudaOps, name, vars(CudaOps)[name]) for name in STANDS_FOR] + [
+    (c, "forward", c.forward) for c in (SandwichNormBlock, PreNormBlock, PagedAttention, GatedFeedForward)] + [
+    (Linear, "__call__", Linear.__call__)]
 
 
 class UniformLayers:
@@ -91,7 +97,10 @@ class UniformLayers:
     return (o.layer_runs and ctx.num_tokens * self.operations_per_token <= MOST_OPERATIONS and o.dtype == torch.bfloat16
             and ctx.max_q_len > 1 and o.fused_qkv_rope and o.direct_library_products and o.gated_tc_pairs
             and not (o.skinny_warps or o.gated_tc_blocks or o.mid_split or o.mid_stages or o.decode_variant)
-            and STANDS_FOR.isdisjoint(vars(o)) and o._uses_tensor_core_attention(self.head_dim, self.group)
+            and STANDS_FOR.isdisjoint(vars(o)) and all(getattr(c, name) is call for c, name, call in OWN_CALLS)
+            and not any("forward" in vars(part) for b in self.blocks for part in (b, b.mixer, b.feed_forward))
+            and all(type(b.mixer.o_proj) is Linear and type(b.feed_forward.down_proj) is Linear for b in self.blocks)
+            and o._uses_tensor_core_attention(self.head_dim, self.group)
             and o._prefill_uses_tcgen05(self.head_dim, self.group, ctx.page_size))
 
   def run(self, h: torch.Tensor, ctx: Any, caches: dict[str, Any]):
